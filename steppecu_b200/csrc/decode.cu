@@ -16,6 +16,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "stpf2_internal.cuh"
 
@@ -318,113 +319,174 @@ constexpr int kSliceBytes = kSliceWords * 4;
 constexpr int kRowStride = kSliceWords + 4;          // words per staged record row (16-byte rows)
 constexpr int kStagedWords = 4 * kTileCols * kRowStride + 32;
 constexpr int kQuadRows = 4 * kTileCols;  // record rows of a quad
-// Two staging buffers, then the quad's row offsets (int64 each).
-constexpr size_t kTransSmemBytes = 2 * kStagedWords * sizeof(uint32_t) + kQuadRows * sizeof(int64_t);
-static_assert((2 * kStagedWords * sizeof(uint32_t)) % 8 == 0, "row table alignment");
+// Two staging buffers, then the quad's row addresses and row slots (8 bytes each).
+constexpr size_t kTransSmemBytes =
+    2 * kStagedWords * sizeof(uint32_t) + kQuadRows * sizeof(uint64_t) + 4 * (kTileCols + 2) * 2 * sizeof(uint32_t);
+static_assert((2 * kStagedWords * sizeof(uint32_t)) % 16 == 0 && kQuadRows % 2 == 0, "row table alignment");
+static_assert(kRowStride >= kSliceWords + 4, "a row's slice spans up to one more granule");
 static_assert(kTransThreads >= kQuadRows && (kQuadRows * (kSliceBytes / 16)) % kTransThreads == 0, "staging split");
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-                 "l"(src)
+// 16 bytes of which the first n come from src and the rest are zero (n = 16: a plain copy).
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "r"(n)
                  : "memory");
 }
 
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-                 "l"(src)
-                 : "memory");
-}
+// The records of a pass: row r's bytes at base + r * pitch, `bytes` of them (the rest of a
+// row is never read), any base and pitch alignment.
+struct RecordView {
+    const uint8_t* base;
+    uint64_t pitch;
+    uint32_t bytes;
+};
 
-// Byte offset of each of the quad's 128 record rows (row sub*32 + r: SNP r of tile 4q+sub,
-// through the row map when rows are kept), or -1 for a row past its tile's SNPs or past the
-// last tile. Computed once per CTA; every slice's staging reads it.
-__device__ __forceinline__ void quad_rows(int64_t* rows, uint64_t pitch, const TileInfo* __restrict__ tiles,
-                                          int64_t n_tiles, int64_t q, const int32_t* __restrict__ row_map) {
+// How the staged words of a row are read back. kGran is the alignment every row start has:
+// 16 (word w of a row is staged word w), 4 (the row starts 0-3 words into its first 16-byte
+// granule) or 1 (it also starts 0-3 bytes into a word, so a word is two staged ones through
+// one PRMT). Copies are whole 16-byte granules in every form: a record file's pitch is
+// ceil(n_ind / 4) bytes, rarely a multiple of 16. Against 4-byte copies of word-aligned rows
+// this took the pass from 1.95 to 1.48 ms at 10,000 samples x 1.15M SNPs and from 428 to 266
+// us at 2,000; rows off a word were first copied into an aligned pitch, 1.09 ms of a 3.87 ms
+// pass at 8,649 samples x 401,113 SNPs, against 0.03 ms for the PRMTs.
+struct RowSlot {
+    uint32_t word;  // staged word of the row's first byte, relative to the slice buffer
+    uint32_t sel;   // PRMT selector of the row's byte shift
+};
+constexpr int kSlotPitch = kTileCols + 2;  // row slots per tile (keeps the tiles on distinct banks)
+
+// Address of each of the quad's 128 record rows (row sub*32 + r: SNP r of tile 4q+sub,
+// through the row map when rows are kept), or 0 for a row past its tile's SNPs or past the
+// last tile, and its slot. Computed once per CTA; every slice's staging reads it.
+template <int kGran>
+__device__ __forceinline__ void quad_rows(uint64_t* rows, RowSlot* slots, const RecordView& v,
+                                          const TileInfo* __restrict__ tiles, int64_t n_tiles, int64_t q,
+                                          const int32_t* __restrict__ row_map) {
     const int row = threadIdx.x;
     if (row >= kQuadRows) return;
     const int sub = row / kTileCols, r = row % kTileCols;
     const int64_t t = 4 * q + sub;
-    int64_t off = -1;
+    uint64_t at = 0;
     if (t < n_tiles) {
         const TileInfo ti = tiles[t];
         if (r < ti.nvalid) {
             const int64_t snp = static_cast<int64_t>(ti.snp0) + r;
-            off = static_cast<int64_t>(row_map ? __ldg(row_map + snp) : snp) * static_cast<int64_t>(pitch);
+            at = reinterpret_cast<uint64_t>(v.base) + static_cast<uint64_t>(row_map ? __ldg(row_map + snp) : snp) * v.pitch;
         }
     }
-    rows[row] = off;
+    rows[row] = at;
+    if constexpr (kGran < 16) {
+        const uint32_t d = static_cast<uint32_t>(at & 15);
+        slots[sub * kSlotPitch + r] =
+            RowSlot{static_cast<uint32_t>(row * kRowStride + sub * 8) + (d >> 2), 0x3210u + (d & 3u) * 0x1111u};
+    }
+}
+
+// Stages one 16-byte granule (number k of the slice, counted from the granule holding the
+// slice's first byte of the row) of a row into d. Only the row's own bytes are read; a row
+// without a record holds code 3 (missing).
+__device__ __forceinline__ void stage_granule(uint32_t* d, const RecordView& v, uint64_t at, uint64_t first) {
+    if (at == 0) {
+        *reinterpret_cast<uint4*>(d) = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+        return;
+    }
+    const uint64_t p = (at & ~uint64_t(15)) + first, end = at + v.bytes;
+    if (p >= end) return;  // past the record: no selected sample reads it
+    if (p < reinterpret_cast<uint64_t>(v.base)) {  // the first record of an unaligned buffer
+        uint8_t* b = reinterpret_cast<uint8_t*>(d);
+        for (int i = 0; i < 16; ++i)
+            if (p + i >= at && p + i < end) b[i] = *reinterpret_cast<const uint8_t*>(p + i);
+        return;
+    }
+    cp_async16(d, reinterpret_cast<const void*>(p), static_cast<uint32_t>(end - p < 16 ? end - p : 16));
 }
 
 // Stages slice `slice` of the quad's 128 records into buf: row (sub, r) at word
 // (sub*32 + r)*kRowStride + sub*8 (the sub*8 skew keeps the threads of one warp on
-// distinct banks when they read it back); bytes past the record and rows without a record
-// (rows[row] < 0) hold code 3 (missing). Thread t copies 16-byte column t % 16 of rows
-// t / 16 + 16 i. kVec16: records and pitch are 16-byte aligned (16-byte copies); otherwise
-// 4-byte aligned (4-byte copies, so a host panel keeps its own pitch on the device).
-template <bool kVec16>
-__device__ __forceinline__ void stage_slice(uint32_t* buf, const uint8_t* __restrict__ records, uint64_t pitch,
-                                            const int64_t* rows, int64_t slice) {
+// distinct banks when they read it back). Thread t copies granule t % 16 of rows
+// t / 16 + 16 i; a row that does not start on a granule takes a 17th.
+template <int kGran>
+__device__ __forceinline__ void stage_slice(uint32_t* buf, const RecordView& v, const uint64_t* rows, int64_t slice) {
     constexpr int kCols16 = kSliceBytes / 16;
     const int k = threadIdx.x % kCols16;
-    const uint64_t b = static_cast<uint64_t>(slice) * kSliceBytes + static_cast<uint64_t>(k) * 16;
+    const uint64_t b = static_cast<uint64_t>(slice) * kSliceBytes;
 #pragma unroll
     for (int i = 0; i < kQuadRows * kCols16 / kTransThreads; ++i) {
         const int row = threadIdx.x / kCols16 + i * (kTransThreads / kCols16);
-        uint32_t* d = buf + row * kRowStride + (row / kTileCols) * 8 + k * 4;
-        const int64_t off = rows[row];
-        if constexpr (kVec16) {
-            if (off >= 0 && b < pitch) cp_async16(d, records + off + b);
-            else *reinterpret_cast<uint4*>(d) = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-        } else {
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                if (off >= 0 && b + 4 * w < pitch) cp_async4(d + w, records + off + b + 4 * w);
-                else d[w] = 0xFFFFFFFFu;
-            }
-        }
+        stage_granule(buf + row * kRowStride + (row / kTileCols) * 8 + k * 4, v, rows[row], b + 16 * k);
+    }
+    if constexpr (kGran < 16) {
+        const int row = threadIdx.x;
+        if (row < kQuadRows)
+            stage_granule(buf + row * kRowStride + (row / kTileCols) * 8 + kSliceWords, v, rows[row], b + kSliceBytes);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// Four consecutive rows' word wl of tile sub (rows 4 rg .. 4 rg + 3).
+template <int kGran>
+__device__ __forceinline__ void staged_words(const uint32_t* srec, const RowSlot* slots, int sub, int rg, int wl,
+                                             uint32_t (&rw)[4]) {
+    if constexpr (kGran == 16) {
+        const uint32_t* base = srec + sub * kTileCols * kRowStride + sub * 8 + wl;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) rw[r] = base[(4 * rg + r) * kRowStride];
+    } else {
+        const uint4* sl = reinterpret_cast<const uint4*>(slots + sub * kSlotPitch + 4 * rg);
+        const uint4 s01 = sl[0], s23 = sl[1];
+        const uint32_t at[4] = {s01.x, s01.z, s23.x, s23.z}, sel[4] = {s01.y, s01.w, s23.y, s23.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t* w = srec + at[r] + wl;
+            rw[r] = kGran == 4 ? w[0] : __byte_perm(w[0], w[1], sel[r]);
+        }
+    }
 }
 
 // Pass 1: SNP-major records -> canonical quads, gathering the selected samples. One CTA per
 // quad of 128 columns walks the record slices of 1024 samples, staging slice s+1 with
 // cp.async while it transposes slice s: thread (word w, tile sub) transposes 16 samples x
 // 32 columns with SWAR 4x4 transposes, and the four threads of a sample write its 32-byte
-// sector together. The first slice also yields each column's centre c_s: the pooled
-// frequency of the called genotypes among the record's first 256 samples, rounded to 1/256
-// (f2 is exact for any per-SNP centre; this one only keeps the operand magnitudes small).
-template <bool kVec16>
+// sector together. With center, the first slice also yields each column's centre c_s: the
+// pooled frequency of the called genotypes among the record's first 256 samples, rounded to
+// 1/256 (f2 is exact for any per-SNP centre; this one only keeps the magnitudes of the split
+// and FP32 operands small; the fixed point and the counts need none).
+template <int kGran>
 __global__ void __launch_bounds__(kTransThreads)
-transpose_pa_kernel(const uint8_t* __restrict__ records, uint64_t pitch, int64_t n_ind,
+transpose_pa_kernel(const RecordView v, int64_t n_ind,
                     const TileInfo* __restrict__ tiles, int64_t n_tiles, const int32_t* __restrict__ pos,
                     int64_t n_sel, int64_t n_slices, uint64_t* __restrict__ canon, double* __restrict__ center,
                     const int32_t* __restrict__ row_map) {
     extern __shared__ __align__(16) uint32_t srec_all[];
     const int64_t q = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t* rows = reinterpret_cast<int64_t*>(srec_all + 2 * kStagedWords);
-    quad_rows(rows, pitch, tiles, n_tiles, q, row_map);
+    uint64_t* rows = reinterpret_cast<uint64_t*>(srec_all + 2 * kStagedWords);
+    RowSlot* slots = reinterpret_cast<RowSlot*>(rows + kQuadRows);
+    quad_rows<kGran>(rows, slots, v, tiles, n_tiles, q, row_map);
     __syncthreads();
-    stage_slice<kVec16>(srec_all, records, pitch, rows, 0);
+    stage_slice<kGran>(srec_all, v, rows, 0);
     for (int64_t slice = 0; slice < n_slices; ++slice) {
         uint32_t* srec = srec_all + (slice & 1) * kStagedWords;
         // One barrier per slice: after it every thread's copies of this slice have landed and
         // every thread is done with the previous slice, whose buffer the next slice refills.
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (slice + 1 < n_slices)
-            stage_slice<kVec16>(srec_all + ((slice + 1) & 1) * kStagedWords, records, pitch, rows, slice + 1);
+        if (slice + 1 < n_slices) stage_slice<kGran>(srec_all + ((slice + 1) & 1) * kStagedWords, v, rows, slice + 1);
 
-        if (slice == 0 && warp < 4) {
+        if (center && slice == 0 && warp < 4) {
             const int sub = warp;
             const int64_t t = 4 * q + sub;
             const int nvalid = t < n_tiles ? tiles[t].nvalid : 0;
-            const int64_t rem = n_ind - static_cast<int64_t>(lane) * 16;
+            const int64_t held = static_cast<int64_t>(v.bytes) * 4;  // samples the records hold
+            const int64_t rem = (n_ind < held ? n_ind : held) - static_cast<int64_t>(lane) * 16;
             const int nv = lane < 16 ? static_cast<int>(rem < 0 ? 0 : (rem < 16 ? rem : 16)) : 0;
             uint32_t vmask = 0;
             for (int m = 0; m < nv; ++m) vmask |= 3u << (8 * (m >> 2) + 6 - 2 * (m & 3));
             for (int r = 0; r < kTileCols; ++r) {
-                const uint32_t x = (nv > 0 ? srec[(sub * kTileCols + r) * kRowStride + sub * 8 + lane] : 0u) & vmask;
+                uint32_t w[4] = {0u, 0u, 0u, 0u};
+                if (nv > 0) staged_words<kGran>(srec, slots, sub, r >> 2, lane, w);
+                const uint32_t x = ((r & 2) ? ((r & 1) ? w[3] : w[2]) : ((r & 1) ? w[1] : w[0])) & vmask;
                 const uint32_t lo = x & 0x55555555u, hi = (x >> 1) & 0x55555555u;
                 const uint32_t miss = lo & hi;
                 const int cnt = __reduce_add_sync(0xffffffffu, __popc(vmask & 0x55555555u) - __popc(miss));
@@ -441,15 +503,13 @@ transpose_pa_kernel(const uint8_t* __restrict__ records, uint64_t pitch, int64_t
             const int64_t rem = n_ind - r0;
             if (rem <= 0) break;
             const int nv = static_cast<int>(rem < 16 ? rem : 16);
-            const uint32_t* base = srec + sub * kTileCols * kRowStride + sub * 8 + wl;
             // y[rg][j]: the 4 x 4 block of SNPs 4rg.. x samples 4j.., transposed so that byte
             // 3 - m holds sample 4j + m's four codes.
             uint32_t y[kTileCols / 4][4];
 #pragma unroll
             for (int rg = 0; rg < kTileCols / 4; ++rg) {
                 uint32_t rw[4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) rw[r] = base[(4 * rg + r) * kRowStride];
+                staged_words<kGran>(srec, slots, sub, rg, wl, rw);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t sel = static_cast<uint32_t>(j) | (static_cast<uint32_t>(j + 4) << 4);
@@ -592,7 +652,8 @@ decode_canon_kernel(const uint64_t* __restrict__ canon, int64_t n_tiles, int64_t
     extern __shared__ uint32_t s_cnt[];
     __shared__ double s_center[4 * kCenterPitch];
     const int64_t q = blockIdx.x;
-    for (int c = threadIdx.x; c < 4 * kTileCols; c += blockDim.x) {
+    // Only the split and FP32 operands are centred.
+    for (int c = threadIdx.x; F != OpFmt::FX && op.planes && c < 4 * kTileCols; c += blockDim.x) {
         const int64_t col = q * 4 * kTileCols + c;
         double cv = 0.5;
         if (col < n_tiles * kTileCols) {
@@ -805,26 +866,55 @@ __global__ void feed_qvn_kernel(const double* __restrict__ Q, const double* __re
 }  // namespace
 
 namespace {
-// The same rule with one warp per 4-byte record word (16 samples): the lanes read the word
-// from 32 records at a time (coalesced across the warps of neighbouring words) and OR
-// their het masks (code 1: low bit set, high bit clear); lanes 0-15 then write the
-// ploidy of the word's selected samples (pos: file row -> selected index, -1 if not).
-__global__ void detect_ploidy_words_kernel(const uint8_t* __restrict__ records, uint64_t pitch, int64_t window,
-                                           int64_t n_ind, const int32_t* __restrict__ pos, uint32_t* __restrict__ sel) {
-    const int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (16 * w >= n_ind) return;  // warp-uniform
-    uint32_t het = 0;
-    for (int64_t s = lane; s < window; s += 32) {
-        const uint32_t x = __ldg(reinterpret_cast<const uint32_t*>(records + s * pitch) + w);
-        het |= (x & 0x55555555u) & ~((x >> 1) & 0x55555555u);
+// Word w (samples 16w .. 16w+15) of a record, any alignment, only the record's own bytes
+// read (the missing ones zero).
+__device__ __forceinline__ uint32_t record_word(const RecordView& v, int64_t s, int64_t w) {
+    const uint8_t* p = v.base + s * static_cast<int64_t>(v.pitch) + 4 * w;
+    const uint32_t d = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p) & 3);
+    if (d == 0 && 4 * w + 4 <= v.bytes) return __ldg(reinterpret_cast<const uint32_t*>(p));
+    if (w == 0 || 4 * w + 8 > v.bytes) {  // the two aligned words may leave the record
+        uint32_t x = 0;
+        for (uint32_t i = 0; i < 4 && 4 * w + i < v.bytes; ++i) x |= static_cast<uint32_t>(__ldg(p + i)) << (8 * i);
+        return x;
     }
-    het = __reduce_or_sync(0xffffffffu, het);
-    const int64_t row = 16 * w + lane;
-    if (lane < 16 && row < n_ind) {
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(p - d);
+    return __byte_perm(__ldg(a), __ldg(a + 1), 0x3210u + d * 0x1111u);
+}
+
+// The same rule over 4-byte record words (16 samples): a CTA takes eight neighbouring words
+// (one sector of a record), its 128 lane groups of eight a stripe of the window each; het
+// masks (code 1: low bit set, high bit clear) are OR-reduced per word, then one thread per
+// sample writes the ploidy of the selected ones (pos: file row -> selected index, -1 if
+// not). A latency-bound pass: eight records per lane in two rounds instead of the 32 of one
+// warp per word (4.1 -> 3.6 us at 400 samples, 11.9 -> 10.4 us at 10,000).
+constexpr int kPlWords = 8, kPlThreads = 1024;
+__global__ void __launch_bounds__(kPlThreads)
+detect_ploidy_words_kernel(const RecordView v, int64_t window, int64_t n_ind, const int32_t* __restrict__ pos,
+                           uint32_t* __restrict__ sel) {
+    __shared__ uint32_t s_het[kPlWords];
+    const int k = threadIdx.x % kPlWords;
+    const int64_t w = static_cast<int64_t>(blockIdx.x) * kPlWords + k;
+    if (threadIdx.x < kPlWords) s_het[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t het = 0;
+    if (16 * w < n_ind) {
+#pragma unroll 4
+        for (int64_t s = threadIdx.x / kPlWords; s < window; s += kPlThreads / kPlWords) {
+            const uint32_t x = record_word(v, s, w);
+            het |= (x & 0x55555555u) & ~((x >> 1) & 0x55555555u);
+        }
+    }
+    het |= __shfl_xor_sync(0xffffffffu, het, 8);
+    het |= __shfl_xor_sync(0xffffffffu, het, 16);
+    if ((threadIdx.x & 31) < kPlWords && het) atomicOr(&s_het[k], het);
+    __syncthreads();
+    const int j = threadIdx.x;  // sample j of the CTA's 128
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * kPlWords * 16 + j;
+    if (j < kPlWords * 16 && row < n_ind) {
         const int32_t g = __ldg(pos + row);
         if (g >= 0) {
-            const bool h = (het >> (8 * (lane >> 2) + 6 - 2 * (lane & 3))) & 1u;
+            const int m = j & 15;
+            const bool h = (s_het[j >> 4] >> (8 * (m >> 2) + 6 - 2 * (m & 3))) & 1u;
             sel[g] = (sel[g] & ~3u) | (h ? 2u : 1u);
         }
     }
@@ -869,14 +959,21 @@ void launch_canonical_to_records(Ctx& c, const uint8_t* packed, uint64_t bpr, in
     c.launches++;
 }
 
-void launch_detect_ploidy_words(Ctx& c, const uint8_t* records, uint64_t pitch, int64_t n_snp, int64_t n_ind,
-                                const int32_t* pos, uint32_t* sel, cudaStream_t s) {
+namespace {
+RecordView record_view(const uint8_t* records, uint64_t pitch, uint64_t bpr, int64_t n_ind) {
+    const uint64_t bytes = std::min<uint64_t>(std::min(bpr, pitch), static_cast<uint64_t>((n_ind + 3) / 4));
+    if (bytes > 0xFFFFFFFFull) fail(STP_INVALID_ARGUMENT, "records longer than 4 GiB");
+    return RecordView{records, pitch, static_cast<uint32_t>(bytes)};
+}
+}  // namespace
+
+void launch_detect_ploidy_words(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_t bpr, int64_t n_snp,
+                                int64_t n_ind, const int32_t* pos, uint32_t* sel, cudaStream_t s) {
     if (n_ind <= 0 || n_snp <= 0) return;
-    if (pitch % 4 != 0 || reinterpret_cast<uintptr_t>(records) % 4 != 0)
-        fail(STP_INVALID_ARGUMENT, "word-wise ploidy detection needs 4-byte aligned records and pitch");
     const int64_t window = n_snp < kPloidyWindow ? n_snp : kPloidyWindow;
-    const int64_t warps = (n_ind + 15) / 16;
-    detect_ploidy_words_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, s>>>(records, pitch, window, n_ind, pos, sel);
+    const int64_t ctas = (n_ind + 16 * kPlWords - 1) / (16 * kPlWords);
+    detect_ploidy_words_kernel<<<static_cast<unsigned>(ctas), kPlThreads, 0, s>>>(record_view(records, pitch, bpr, n_ind),
+                                                                                  window, n_ind, pos, sel);
     STPF2_CUDA(cudaGetLastError());
     c.launches++;
 }
@@ -892,27 +989,37 @@ void launch_detect_ploidy_pa(Ctx& c, const uint8_t* records, uint64_t pitch, int
     c.launches++;
 }
 
-void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, int64_t n_ind, const TileInfo* tiles,
-                         int64_t n_tiles, const int32_t* pos, int64_t n_sel, uint64_t* canon, double* center,
-                         cudaStream_t s, const int32_t* row_map) {
-    if (n_tiles <= 0) return;
-    const uint64_t align = pitch | static_cast<uint64_t>(reinterpret_cast<uintptr_t>(records));
-    if (align % 4 != 0) fail(STP_INVALID_ARGUMENT, "transpose: genotype records need a 4-byte aligned pitch");
-    const bool vec16 = align % 16 == 0;
-    const int64_t n_quads = (n_tiles + 3) / 4;
-    const int64_t n_slices = std::max<int64_t>(1, (n_ind + kSliceWords * 16 - 1) / (kSliceWords * 16));
-    static bool attr_set[2][64] = {};  // per form and device ordinal
-    if (c.device < 0 || c.device >= 64 || !attr_set[vec16][c.device]) {
-        STPF2_CUDA(cudaFuncSetAttribute(vec16 ? transpose_pa_kernel<true> : transpose_pa_kernel<false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTransSmemBytes)));
-        if (c.device >= 0 && c.device < 64) attr_set[vec16][c.device] = true;
+namespace {
+template <int kGran>
+void transpose_gran(Ctx& c, unsigned n_quads, const RecordView& v, int64_t n_ind, const TileInfo* tiles, int64_t n_tiles,
+                    const int32_t* pos, int64_t n_sel, int64_t n_slices, uint64_t* canon, double* center,
+                    const int32_t* row_map, cudaStream_t s) {
+    static std::atomic<bool> attr_set[64] = {};  // per device ordinal
+    if (c.device < 0 || c.device >= 64 || !attr_set[c.device]) {
+        STPF2_CUDA(cudaFuncSetAttribute(transpose_pa_kernel<kGran>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(kTransSmemBytes)));
+        if (c.device >= 0 && c.device < 64) attr_set[c.device] = true;
     }
-    if (vec16)
-        transpose_pa_kernel<true><<<static_cast<unsigned>(n_quads), kTransThreads, kTransSmemBytes, s>>>(
-            records, pitch, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map);
+    transpose_pa_kernel<kGran><<<n_quads, kTransThreads, kTransSmemBytes, s>>>(v, n_ind, tiles, n_tiles, pos, n_sel,
+                                                                               n_slices, canon, center, row_map);
+}
+}  // namespace
+
+void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_t bpr, int64_t n_ind,
+                         const TileInfo* tiles, int64_t n_tiles, const int32_t* pos, int64_t n_sel, uint64_t* canon,
+                         double* center, cudaStream_t s, const int32_t* row_map) {
+    if (n_tiles <= 0) return;
+    const RecordView v = record_view(records, pitch, bpr, n_ind);
+    // Every row starts where the pitch and the base put it: the form is their common alignment.
+    const uint64_t align = pitch | static_cast<uint64_t>(reinterpret_cast<uintptr_t>(records));
+    const unsigned n_quads = static_cast<unsigned>((n_tiles + 3) / 4);
+    const int64_t n_slices = std::max<int64_t>(1, (n_ind + kSliceWords * 16 - 1) / (kSliceWords * 16));
+    if (align % 16 == 0)
+        transpose_gran<16>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s);
+    else if (align % 4 == 0)
+        transpose_gran<4>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s);
     else
-        transpose_pa_kernel<false><<<static_cast<unsigned>(n_quads), kTransThreads, kTransSmemBytes, s>>>(
-            records, pitch, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map);
+        transpose_gran<1>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s);
     STPF2_CUDA(cudaGetLastError());
     c.launches++;
 }
@@ -1099,7 +1206,8 @@ void launch_decode_canon(Ctx& c, const CanonDecodeArgs& a, cudaStream_t s) {
 #define STPF2_DECODE_LAUNCH(F)                                                                      \
     (a.umap ? decode_canon_kernel<F, true><<<grid, kDecThreads2, kDecSmemBytes, s>>>(STPF2_DECODE_ARGS) \
             : decode_canon_kernel<F, false><<<grid, kDecThreads2, kDecSmemBytes, s>>>(STPF2_DECODE_ARGS))
-    if (a.umap && !a.center_snp) fail(STP_INVALID_ARGUMENT, "shared-canonical decode needs per-SNP centres");
+    if (a.op.fmt != OpFmt::FX && a.op.planes && !(a.umap ? a.center_snp : a.center))
+        fail(STP_INVALID_ARGUMENT, "decode of centred operands needs the centres");
     switch (a.op.fmt) {
         case OpFmt::F32: STPF2_DECODE_LAUNCH(OpFmt::F32); break;
         case OpFmt::BF16: STPF2_DECODE_LAUNCH(OpFmt::BF16); break;

@@ -102,7 +102,7 @@ size_t noalloc_scratch_bytes(int64_t n_snp, int64_t n_ind, int64_t n_sel, int P,
     return b;
 }
 
-void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, int64_t n_snp, int64_t n_ind,
+void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, uint64_t bpr, int64_t n_snp, int64_t n_ind,
                            const int64_t* sel_rows, int64_t n_sel, const int64_t* pop_offsets, int P,
                            const int32_t* sample_ploidy, int mode_ploidy, bool detect, int32_t* d_ac2,
                            int32_t* d_n, cudaStream_t s) {
@@ -153,8 +153,8 @@ void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, int
         n_snp, n_tiles, d_tiles, d_col_snp, d_po64, d_po32, P);
     STPF2_CUDA(cudaGetLastError());
     c.launches++;
-    if (detect) launch_detect_ploidy_words(c, d_records, pitch, n_snp, n_ind, d_pos, d_desc, s);
-    launch_transpose_pa(c, d_records, pitch, n_ind, d_tiles, n_tiles, d_pos, n_sel_pad, d_canon, d_center, s);
+    if (detect) launch_detect_ploidy_words(c, d_records, pitch, bpr, n_snp, n_ind, d_pos, d_desc, s);
+    launch_transpose_pa(c, d_records, pitch, bpr, n_ind, d_tiles, n_tiles, d_pos, n_sel_pad, d_canon, nullptr, s);
     CanonDecodeArgs a;
     a.canon = d_canon;
     a.n_tiles = n_tiles;
@@ -162,7 +162,6 @@ void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, int
     a.sel = d_desc;
     a.pop_off = d_po32;
     a.P = P;
-    a.center = d_center;
     a.col_snp = d_col_snp;
     a.op.planes = nullptr;  // counts only
     a.cnt_ac2 = d_ac2;

@@ -174,7 +174,7 @@ struct Plan {
     int precision = 0;
     bool detect = false;
     BlockLayout L;
-    DevBuf sel, pop_off, pos, tiles, col_snp, rec_n, rec_nm1, canon, center, blocks, items, own_planes, repitched;
+    DevBuf sel, pop_off, pos, tiles, col_snp, rec_n, rec_nm1, canon, center, blocks, items, own_planes;
     DevBuf fold_order;  // per 64-population group, local indices largest first (null: all equal)
     DevBuf fx_table;    // FX: the term table of every (n, a2) (OperandPlanes::fx_table)
     DevBuf row_map;     // kept SNP -> record row (empty: SNP s is record s)
@@ -183,8 +183,8 @@ struct Plan {
     double* center_ptr = nullptr;
     int64_t n_ind = 0, n_tiles = 0, n_sel_pad = 0;
     int n_items = 0;
-    bool repitch = false;
-    uint64_t src_pitch = 0, bpr = 0;
+    bool words = true;  // records and pitch 4-byte aligned, whole rows within the pitch
+    uint64_t bpr = 0;
     OperandPlanes op;
     UmmaPlan* umma = nullptr;
     // Timing: three events per run (start, after decode, after contraction), one set per
@@ -348,17 +348,10 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
         p->center_ptr = eb.as<double>();
     }
 
-    // The transpose reads records with 4-byte (16-byte when aligned so) copies: records of
-    // a pitch that is not a multiple of 4 are copied once per run into a 16-byte pitch.
+    // The decode reads records of any pitch and alignment in place.
     p->bpr = r.geno.bytes_per_record;
-    p->src_pitch = pitch;
-    const uint64_t need_bytes = static_cast<uint64_t>((r.geno.n_ind + 63) / 64) * 16;
-    p->repitch = (pitch % 4 != 0) || pitch < static_cast<uint64_t>((r.geno.n_ind + 3) / 4) ||
-                 (r.geno.on_device && reinterpret_cast<uintptr_t>(r.geno.records) % 4 != 0);
-    if (p->repitch) {
-        p->pitch = (std::max<uint64_t>(r.geno.bytes_per_record, need_bytes) + 15) / 16 * 16;
-        p->repitched.reserve(std::max<size_t>(static_cast<size_t>(p->pitch) * p->n_rec, 64));
-    }
+    p->words = pitch % 4 == 0 && pitch >= static_cast<uint64_t>((r.geno.n_ind + 3) / 4) &&
+               !(r.geno.on_device && reinterpret_cast<uintptr_t>(r.geno.records) % 4 != 0);
     upload(p->blocks, p->L.blocks, s);
     if (counts_only) return p;  // decode to counts only: no operand planes, no contraction
 
@@ -401,16 +394,15 @@ void launch_decode(Plan& p, const uint8_t* d_records, int32_t* cnt_ac2, int32_t*
     if (p.n_snp <= 0) return;
     if (t1 < 0) t1 = p.n_tiles;
     const uint8_t* rec = d_records;
-    if (p.repitch) {
-        STPF2_CUDA(cudaMemcpy2DAsync(p.repitched.ptr, p.pitch, d_records, p.src_pitch, p.bpr,
-                                     static_cast<size_t>(p.n_rec), cudaMemcpyDeviceToDevice, s));
-        rec = p.repitched.as<uint8_t>();
-    }
+    if (p.words && reinterpret_cast<uintptr_t>(rec) % 4 != 0)  // a plan built for aligned records
+        fail(STP_INVALID_ARGUMENT, "transpose: genotype records need a 4-byte aligned pitch");
     if (p.detect && detect)
-        launch_detect_ploidy_words(c, rec, p.pitch, p.n_rec, p.n_ind, p.pos.as<int32_t>(), p.sel.as<uint32_t>(), s);
+        launch_detect_ploidy_words(c, rec, p.pitch, p.bpr, p.n_rec, p.n_ind, p.pos.as<int32_t>(), p.sel.as<uint32_t>(), s);
     if (t1 <= t0) return;
-    launch_transpose_pa(c, rec, p.pitch, p.n_ind, p.tiles.as<TileInfo>() + t0, t1 - t0, p.pos.as<int32_t>(),
-                        p.n_sel_pad, p.canon_ptr, p.center_ptr + t0 * kTileK, s, p.row_map.as<int32_t>());
+    const bool counts = cnt_ac2 || cnt_packed;
+    double* center = p.op.fmt == OpFmt::FX || counts ? nullptr : p.center_ptr + t0 * kTileK;
+    launch_transpose_pa(c, rec, p.pitch, p.bpr, p.n_ind, p.tiles.as<TileInfo>() + t0, t1 - t0, p.pos.as<int32_t>(),
+                        p.n_sel_pad, p.canon_ptr, center, s, p.row_map.as<int32_t>());
     CanonDecodeArgs a;
     a.canon = p.canon_ptr;
     a.n_tiles = t1 - t0;
@@ -418,7 +410,7 @@ void launch_decode(Plan& p, const uint8_t* d_records, int32_t* cnt_ac2, int32_t*
     a.sel = p.sel.as<uint32_t>();
     a.pop_off = p.pop_off.as<int32_t>();
     a.P = p.P;
-    a.center = p.center_ptr + t0 * kTileK;
+    a.center = center;
     a.rec_n = p.rec_n.as<double>();
     a.rec_nm1 = p.rec_nm1.as<double>();
     a.col_snp = p.col_snp.as<int32_t>() + t0 * kTileK;
@@ -468,27 +460,15 @@ void copy_block_sizes(const BlockLayout& L, int32_t* out) {
     for (int b = 0; b < L.n_block; ++b) out[b] = L.blocks[b].k;
 }
 
-// Device pitch for host records: their own pitch when the transpose can read it (a
-// multiple of 4 bytes), so the upload is one contiguous copy; else rounded up to 16.
-uint64_t device_pitch(const stp_geno_view& g) {
-    const uint64_t hp = g.pitch ? g.pitch : g.bytes_per_record;
-    return hp % 4 == 0 ? hp : (g.bytes_per_record + 15) / 16 * 16;
-}
-
-// Copies record rows [s0, s0 + n) from the host into d (pitch dp) on stream st: one
-// contiguous copy when the pitches agree (the last row only up to bytes_per_record, which
-// is all a host buffer is sure to hold), else a pitched copy.
-void upload_rows(const stp_geno_view& g, uint8_t* d, uint64_t dp, int64_t s0, int64_t n, cudaStream_t st) {
+// Copies record rows [s0, s0 + n) from the host into d, at the records' own pitch hp, on
+// stream st: one contiguous copy (the last row only up to bytes_per_record, which is all a
+// host buffer is sure to hold). Rows of any pitch go as they are: a row-by-row copy into an
+// aligned pitch ran at 4 GB/s for 375-byte rows, the contiguous one at the link's 50.
+void upload_rows(const stp_geno_view& g, uint8_t* d, uint64_t hp, int64_t s0, int64_t n, cudaStream_t st) {
     if (n <= 0) return;
-    const uint64_t hp = g.pitch ? g.pitch : g.bytes_per_record;
-    if (hp == dp) {
-        const size_t bytes = static_cast<size_t>(n - 1) * hp + g.bytes_per_record;
-        STPF2_CUDA(cudaMemcpyAsync(d + s0 * static_cast<int64_t>(dp), g.records + s0 * static_cast<int64_t>(hp), bytes,
-                                   cudaMemcpyHostToDevice, st));
-    } else {
-        STPF2_CUDA(cudaMemcpy2DAsync(d + s0 * static_cast<int64_t>(dp), dp, g.records + s0 * static_cast<int64_t>(hp), hp,
-                                     g.bytes_per_record, static_cast<size_t>(n), cudaMemcpyHostToDevice, st));
-    }
+    const size_t bytes = static_cast<size_t>(n - 1) * hp + std::min(hp, g.bytes_per_record);
+    STPF2_CUDA(cudaMemcpyAsync(d + s0 * static_cast<int64_t>(hp), g.records + s0 * static_cast<int64_t>(hp), bytes,
+                               cudaMemcpyHostToDevice, st));
 }
 
 // Runs f(i) for i in [0, n) on up to hardware_concurrency threads; rethrows the first error.
@@ -894,11 +874,10 @@ void extract_one(Ctx& c, const stp_f2_request& r, stp_f2_output& o) {
     uint64_t dp = 0;
     if (host_in) {
         need(r.geno.records != nullptr, "records is NULL");
-        dp = device_pitch(r.geno);
+        dp = pitch;
         c.ws_records.reserve(static_cast<size_t>(dp) * r.geno.n_snp);
         if (!pipelined) upload_rows(r.geno, c.ws_records.as<uint8_t>(), dp, 0, r.geno.n_snp, s);
         d_rec = c.ws_records.as<uint8_t>();
-        pitch = dp;
     }
     // A repeated request reuses its plan (whose operand planes already sit in the
     // workspace); otherwise the operand planes borrow the context's grow-only workspace.
@@ -911,7 +890,7 @@ void extract_one(Ctx& c, const stp_f2_request& r, stp_f2_output& o) {
     }
     if (o.block_sizes) copy_block_sizes(p->L, o.block_sizes);
     const size_t out_elems = static_cast<size_t>(std::max(r.n_pop, 0)) * std::max(r.n_pop, 0) * std::max(r.n_block, 0);
-    if (pipelined && p->umma && !p->repitch && out_elems) {
+    if (pipelined && p->umma && out_elems) {
         STPF2_CUDA(cudaStreamSynchronize(s));  // the plan's tables are uploaded on s
         SlabTarget t;
         t.f2 = o.f2;
@@ -1043,29 +1022,16 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
     need(n_ind > 0, "n_ind must be positive");
     need(g.bytes_per_record > 0, "bytes_per_record is 0");
     need(M < INT_MAX, "too many SNPs");
-    uint64_t pitch = g.pitch ? g.pitch : g.bytes_per_record;
+    const uint64_t pitch = g.pitch ? g.pitch : g.bytes_per_record;
     need(pitch >= g.bytes_per_record, "pitch < bytes_per_record");
     const int prec = reqs[idx[0]].precision;
     const OpFmt fmt = fmt_of(prec);
 
-    // Records on the device at a pitch the transpose reads (a multiple of 4 bytes).
     const uint8_t* d_rec = g.records;
-    DevBuf repitched;
     if (!g.on_device) {
-        const uint64_t dp = device_pitch(g);
-        c.ws_records.reserve(static_cast<size_t>(dp) * M);
-        upload_rows(g, c.ws_records.as<uint8_t>(), dp, 0, M, s);
+        c.ws_records.reserve(static_cast<size_t>(pitch) * M);
+        upload_rows(g, c.ws_records.as<uint8_t>(), pitch, 0, M, s);
         d_rec = c.ws_records.as<uint8_t>();
-        pitch = dp;
-    } else if (pitch % 4 != 0 || pitch < static_cast<uint64_t>((n_ind + 3) / 4) ||
-               reinterpret_cast<uintptr_t>(g.records) % 4 != 0) {
-        const uint64_t need_bytes = static_cast<uint64_t>((n_ind + 63) / 64) * 16;
-        const uint64_t dp = (std::max<uint64_t>(g.bytes_per_record, need_bytes) + 15) / 16 * 16;
-        repitched.reserve(static_cast<size_t>(dp) * M);
-        STPF2_CUDA(cudaMemcpy2DAsync(repitched.ptr, dp, g.records, pitch, g.bytes_per_record, static_cast<size_t>(M),
-                                     cudaMemcpyDeviceToDevice, s));
-        d_rec = repitched.as<uint8_t>();
-        pitch = dp;
     }
 
     // The union of the selected samples, in file order.
@@ -1129,8 +1095,9 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
     launch_timestamp(c, d_t0, s);
     launch_layout_tables(c, reinterpret_cast<BlockInfo*>(U + o_one), reinterpret_cast<int64_t*>(U + o_zero), 1,
                          n_utiles * kTileK, d_cols_u, d_tiles_u, s);
-    if (any_auto) launch_detect_ploidy_words(c, d_rec, pitch, M, n_ind, d_pos_u, d_desc_u, s);
-    launch_transpose_pa(c, d_rec, pitch, n_ind, d_tiles_u, n_utiles, d_pos_u, n_u_pad, d_canon_u, d_center_u, s);
+    if (any_auto) launch_detect_ploidy_words(c, d_rec, pitch, g.bytes_per_record, M, n_ind, d_pos_u, d_desc_u, s);
+    launch_transpose_pa(c, d_rec, pitch, g.bytes_per_record, n_ind, d_tiles_u, n_utiles, d_pos_u, n_u_pad, d_canon_u,
+                        fmt == OpFmt::FX ? nullptr : d_center_u, s);
 
     // Host tables of every request, in parallel, while the device runs the shared passes.
     std::vector<BatchMember> mem(idx.size());
@@ -1447,11 +1414,9 @@ stp_status stp_decode_counts(stp_ctx* ctx, const stp_geno_view* geno, const int6
         uint64_t pitch = geno->pitch ? geno->pitch : geno->bytes_per_record;
         DevBuf rec;
         if (!geno->on_device) {
-            const uint64_t dp = device_pitch(*geno);
-            rec.reserve(static_cast<size_t>(dp) * geno->n_snp);
-            upload_rows(*geno, rec.as<uint8_t>(), dp, 0, geno->n_snp, s);
+            rec.reserve(static_cast<size_t>(pitch) * geno->n_snp);
+            upload_rows(*geno, rec.as<uint8_t>(), pitch, 0, geno->n_snp, s);
             d_rec = rec.as<uint8_t>();
-            pitch = dp;
         }
         std::unique_ptr<Plan> p = build_plan(*ctx, r, pitch, nullptr);
         const size_t cnt = static_cast<size_t>(n_pop) * geno->n_snp;
@@ -1525,11 +1490,9 @@ stp_status stp_snp_keep_mask(stp_ctx* ctx, const stp_geno_view* geno, const int6
             uint64_t pitch = geno->pitch ? geno->pitch : geno->bytes_per_record;
             DevBuf rec;
             if (!geno->on_device) {
-                const uint64_t dp = device_pitch(*geno);
-                rec.reserve(static_cast<size_t>(dp) * M);
-                upload_rows(*geno, rec.as<uint8_t>(), dp, 0, M, s);
+                rec.reserve(static_cast<size_t>(pitch) * M);
+                upload_rows(*geno, rec.as<uint8_t>(), pitch, 0, M, s);
                 d_rec = rec.as<uint8_t>();
-                pitch = dp;
             }
             std::unique_ptr<Plan> p = build_plan(*ctx, r, pitch, nullptr, false, /*counts_only=*/true);
             DevBuf cnt;
@@ -1688,7 +1651,7 @@ stp_status stp_decode_counts_noalloc(stp_ctx* ctx, const stp_geno_view* geno, co
             else need(false, "unknown ploidy_mode");
         }
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-        noalloc_decode_counts(*ctx, geno->records, pitch, geno->n_snp, geno->n_ind, sel_rows, n_sel, pop_offsets,
+        noalloc_decode_counts(*ctx, geno->records, pitch, geno->bytes_per_record, geno->n_snp, geno->n_ind, sel_rows, n_sel, pop_offsets,
                               n_pop, sample_ploidy, mode_pl, detect, d_ac2, d_n, s);
     });
 }
@@ -1905,9 +1868,8 @@ stp_status stp_f2_extract_streamed(stp_ctx* ctx, const stp_f2_request* req, stp_
         need(pitch >= r.geno.bytes_per_record, "pitch < bytes_per_record");
         need(r.geno.records != nullptr || r.geno.n_snp == 0, "records is NULL");
         uint8_t* d_rec = const_cast<uint8_t*>(r.geno.records);
-        uint64_t dp = pitch;
+        const uint64_t dp = pitch;
         if (!r.geno.on_device && r.geno.n_snp > 0) {
-            dp = device_pitch(r.geno);
             c.ws_records.reserve(static_cast<size_t>(dp) * r.geno.n_snp);
             d_rec = c.ws_records.as<uint8_t>();
         }
@@ -1916,7 +1878,7 @@ stp_status stp_f2_extract_streamed(stp_ctx* ctx, const stp_f2_request* req, stp_
             c.ws_misc.reserve(operand_plane_bytes(fmt_of(r.precision), std::max(r.n_pop, 1), probe.ld));
         }
         std::unique_ptr<Plan> p = build_plan(c, r, dp, c.ws_misc.ptr, true);
-        need(!p->repitch, "streamed extraction of device records needs a 4-byte aligned pitch");
+        need(p->words || !r.geno.on_device, "streamed extraction of device records needs a 4-byte aligned pitch");
         if (block_sizes) copy_block_sizes(p->L, block_sizes);
         STPF2_CUDA(cudaStreamSynchronize(c.stream));
         SlabTarget t;

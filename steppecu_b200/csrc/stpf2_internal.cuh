@@ -311,7 +311,7 @@ struct CanonDecodeArgs {
     const uint32_t* sel = nullptr;     // [n_sel] descriptors (ploidy in the low bits)
     const int32_t* pop_off = nullptr;  // [P+1]
     int P = 0;
-    const double* center = nullptr;    // [ld] per-column centre (a multiple of 1/256)
+    const double* center = nullptr;    // [ld] per-column centre (a multiple of 1/256); split / FP32 planes only
     const double* rec_n = nullptr;     // [n_max+1] 1/n (0 at n = 0)
     const double* rec_nm1 = nullptr;   // [n_max+1] 1/max(n-1, 1)
     const int32_t* col_snp = nullptr;  // [ld] SNP of each column, -1 for padding
@@ -335,16 +335,18 @@ struct CanonDecodeArgs {
     const int32_t* fold_order = nullptr;
 };
 
-// Ploidy detection over 4-byte record words (records and pitch 4-byte aligned); pos maps
-// file rows to selected indices (-1: not selected), each row selected once.
-void launch_detect_ploidy_words(Ctx& c, const uint8_t* records, uint64_t pitch, int64_t n_snp, int64_t n_ind,
-                                const int32_t* pos, uint32_t* sel, cudaStream_t s);
+// Ploidy detection over 4-byte record words (records of any pitch and alignment, `bpr` bytes
+// each); pos maps file rows to selected indices (-1: not selected), each row selected once.
+void launch_detect_ploidy_words(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_t bpr, int64_t n_snp,
+                                int64_t n_ind, const int32_t* pos, uint32_t* sel, cudaStream_t s);
 void launch_detect_ploidy_pa(Ctx& c, const uint8_t* records, uint64_t pitch, int64_t n_snp,
                              uint32_t* sel, int64_t n_sel, cudaStream_t s);
-// row_map (optional): record row of every SNP index the tiles name (a kept-SNP compaction).
-void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, int64_t n_ind, const TileInfo* tiles,
-                         int64_t n_tiles, const int32_t* pos, int64_t n_sel, uint64_t* canon, double* center,
-                         cudaStream_t s, const int32_t* row_map = nullptr);
+// Records of any pitch and alignment, `bpr` bytes each. center null: no centres (fixed-point
+// operands and counts read none). row_map (optional): record row of every SNP index the
+// tiles name (a kept-SNP compaction).
+void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_t bpr, int64_t n_ind,
+                         const TileInfo* tiles, int64_t n_tiles, const int32_t* pos, int64_t n_sel, uint64_t* canon,
+                         double* center, cudaStream_t s, const int32_t* row_map = nullptr);
 // Canonical individual-major tile -> SNP-major records (pitch >= ceil(n_ind / 4)).
 void launch_canonical_to_records(Ctx& c, const uint8_t* packed, uint64_t bpr, int64_t n_snp, int64_t n_ind,
                                  uint8_t* records, uint64_t pitch, cudaStream_t s);
@@ -478,7 +480,7 @@ void mirror_lower_tiles(double* S, int64_t P, int64_t T);
 // device array of kNoAllocScratchBytes.
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;
 size_t noalloc_scratch_bytes(int64_t n_snp, int64_t n_ind, int64_t n_sel, int P, bool copy_ploidy);
-void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, int64_t n_snp, int64_t n_ind,
+void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, uint64_t bpr, int64_t n_snp, int64_t n_ind,
                            const int64_t* sel_rows, int64_t n_sel, const int64_t* pop_offsets, int P,
                            const int32_t* sample_ploidy, int mode_ploidy, bool detect, int32_t* d_ac2,
                            int32_t* d_n, cudaStream_t s);

@@ -1,11 +1,10 @@
 // steppecu_b200/csrc/jackknife.cu
 //
-// FP64 block jackknife over per-block values, one thread per item (pop pair): the
-// block-size-weighted total, leave-one-out values, their weighted mean and the AT2
-// jackknife variance of cpu_backend.cpp:2674-2720 (compute_loo_and_total) and
-// :2273-2306 (jackknife_diag). The reference sums in long double; the device has no
-// wider type, so every sum here is a compensated (two-sum) FP64 sum, whose error stays
-// at the level of one FP64 rounding of the result.
+// FP64 block jackknife over per-block values: the block-size-weighted total, leave-one-out
+// values, their weighted mean and the AT2 jackknife variance of cpu_backend.cpp:2674-2720
+// (compute_loo_and_total) and :2273-2306 (jackknife_diag). The reference sums in long
+// double; the device has no wider type, so every sum here is a compensated (two-sum) FP64
+// sum, whose error stays at the level of one FP64 rounding of the result.
 #include "stpf2_internal.cuh"
 
 namespace stpf2 {
@@ -22,43 +21,100 @@ struct CSum {  // Neumaier compensated sum
     __device__ double value() const { return s + c; }
 };
 
-__global__ void jackknife_kernel(const double* __restrict__ x, const int32_t* __restrict__ bl,
-                                 int64_t m, int nb, double n, double* est, double* var) {
-    const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= m) return;
+// One CTA per 32 items (a lane each, so every load is 256 contiguous bytes); its 16 warps
+// take the blocks round robin, and each sum is combined over the warps through shared
+// memory, the compensations included. A thread per item walked all blocks alone: 40 CTAs and
+// a serial chain of compensated adds and divisions for 5,000 items x 714 blocks, 860 us
+// against 176 us. What depends on the block alone (its weight, n / bl and the root) is computed
+// once per warp and block, one block per lane, and shuffled.
+constexpr int kJkWarps = 16;
+
+struct JkBlock {
+    double bl, rel, h, root;  // bl, bl / n, n / bl, sqrt(n / bl - 1)
+};
+
+__device__ __forceinline__ double jk_total(CSum v, double (*s_part)[kJkWarps][32], int warp, int lane) {
+    __syncthreads();  // the previous total has been read
+    s_part[0][warp][lane] = v.s;
+    s_part[1][warp][lane] = v.c;
+    __syncthreads();
+    CSum t;
+#pragma unroll
+    for (int w = 0; w < kJkWarps; ++w) {
+        t.add(s_part[0][w][lane]);
+        t.add(s_part[1][w][lane]);
+    }
+    return t.value();
+}
+
+// f(block, value) for every block of this warp, in block order.
+template <bool kRoot, class F>
+__device__ __forceinline__ void jk_blocks(const double* __restrict__ x, const int32_t* __restrict__ bl, int64_t m, int nb,
+                                          double n, int64_t k, bool real, int warp, int lane, F&& f) {
+    for (int b0 = warp; b0 < nb; b0 += 32 * kJkWarps) {
+        JkBlock mine{1.0, 0.0, 0.0, 0.0};
+        const int bm = b0 + lane * kJkWarps;
+        if (bm < nb) {
+            mine.bl = static_cast<double>(bl[bm]);
+            mine.rel = mine.bl / n;
+            if constexpr (kRoot) {
+                mine.h = n / mine.bl;
+                mine.root = sqrt(mine.h - 1.0);
+            }
+        }
+        const int cnt = min(32, (nb - b0 + kJkWarps - 1) / kJkWarps);
+#pragma unroll 4
+        for (int j = 0; j < cnt; ++j) {
+            JkBlock t;
+            t.bl = __shfl_sync(0xffffffffu, mine.bl, j);
+            t.rel = __shfl_sync(0xffffffffu, mine.rel, j);
+            if constexpr (kRoot) {
+                t.h = __shfl_sync(0xffffffffu, mine.h, j);
+                t.root = __shfl_sync(0xffffffffu, mine.root, j);
+            }
+            f(t, real ? x[k + m * (b0 + j * kJkWarps)] : 0.0);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(32 * kJkWarps)
+jackknife_kernel(const double* __restrict__ x, const int32_t* __restrict__ bl, int64_t m, int nb, double n, double* est,
+                 double* var) {
+    __shared__ double s_part[2][kJkWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + lane;
+    const bool real = k < m;
     CSum num;
-    for (int b = 0; b < nb; ++b) num.add(x[k + m * b] * static_cast<double>(bl[b]));
-    const double tot = num.value() / n;
+    jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) { num.add(v * t.bl); });
+    const double tot = jk_total(num, s_part, warp, lane) / n;
     // Weighted mean of the leave-one-out values (weights 1 - bl/n).
     CSum wnum, wden, wbl;
-    for (int b = 0; b < nb; ++b) {
-        const double rel = static_cast<double>(bl[b]) / n;
-        const double loo = (tot - x[k + m * b] * rel) / (1.0 - rel);
-        const double w = 1.0 - rel;
+    jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
+        const double w = 1.0 - t.rel;
+        const double loo = (tot - v * t.rel) / w;
         wnum.add(loo * w);
         wden.add(w);
-        wbl.add(loo * static_cast<double>(bl[b]));
-    }
-    const double totline = wnum.value() / wden.value();
+        wbl.add(loo * t.bl);
+    });
+    const double totline = jk_total(wnum, s_part, warp, lane) / jk_total(wden, s_part, warp, lane);
+    const double wbl_n = jk_total(wbl, s_part, warp, lane) / n;
     CSum diff;
-    for (int b = 0; b < nb; ++b) {
-        const double rel = static_cast<double>(bl[b]) / n;
-        const double loo = (tot - x[k + m * b] * rel) / (1.0 - rel);
-        diff.add(totline - loo);
-    }
-    const double term1 = (diff.value() / nb) * nb;
-    const double e = term1 + wbl.value() / n;
+    jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
+        diff.add(totline - (tot - v * t.rel) / (1.0 - t.rel));
+    });
+    const double term1 = (jk_total(diff, s_part, warp, lane) / nb) * nb;
+    const double e = term1 + wbl_n;
     CSum acc;
-    for (int b = 0; b < nb; ++b) {
-        const double bl_d = static_cast<double>(bl[b]);
-        const double rel = bl_d / n;
-        const double loo = (tot - x[k + m * b] * rel) / (1.0 - rel);
-        const double h = n / bl_d;
-        const double xtau = (e * h - loo * (h - 1.0) - totline) / sqrt(h - 1.0);
+    jk_blocks<true>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
+        const double loo = (tot - v * t.rel) / (1.0 - t.rel);
+        const double xtau = (e * t.h - loo * (t.h - 1.0) - totline) / t.root;
         acc.add(xtau * xtau);
+    });
+    const double sum = jk_total(acc, s_part, warp, lane);
+    if (real && warp == 0) {
+        est[k] = e;
+        var[k] = sum / nb;
     }
-    est[k] = e;
-    var[k] = acc.value() / nb;
 }
 
 // survivor_blocks (cpu_backend.cpp:124-151): one CTA per block; keep[b] = 0 when block b
@@ -118,18 +174,14 @@ __global__ void fstat_assemble_kernel(const double* __restrict__ f2, int64_t P, 
 
 }  // namespace
 
-void launch_jackknife(Ctx& c, const double* x, const int32_t* block_sizes, int64_t m, int nb,
-                      double* est, double* var, cudaStream_t s) {
+void launch_jackknife(Ctx& c, const double* x, const int32_t* block_sizes, const std::vector<int32_t>& sizes,
+                      int64_t m, double* est, double* var, cudaStream_t s) {
+    const int nb = static_cast<int>(sizes.size());
     if (m <= 0 || nb <= 0) return;
     // n = sum of block sizes (exact in FP64 for any realistic SNP count).
-    std::vector<int32_t> h(static_cast<size_t>(nb));
-    STPF2_CUDA(cudaMemcpyAsync(h.data(), block_sizes, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
-    STPF2_CUDA(cudaStreamSynchronize(s));
     double n = 0.0;
-    for (int32_t v : h) n += static_cast<double>(v);
-    const int threads = 128;
-    jackknife_kernel<<<static_cast<unsigned>((m + threads - 1) / threads), threads, 0, s>>>(
-        x, block_sizes, m, nb, n, est, var);
+    for (int32_t v : sizes) n += static_cast<double>(v);
+    jackknife_kernel<<<static_cast<unsigned>((m + 31) / 32), 32 * kJkWarps, 0, s>>>(x, block_sizes, m, nb, n, est, var);
     STPF2_CUDA(cudaGetLastError());
     c.launches++;
 }

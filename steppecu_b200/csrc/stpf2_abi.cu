@@ -2018,7 +2018,7 @@ stp_status stp_fstats(stp_ctx* ctx, const double* f2, const double* vpair, const
         STPF2_CUDA(cudaMemcpyAsync(d_bl, bl.data(), bl.size() * 4, cudaMemcpyHostToDevice, s));
         STPF2_CUDA(cudaMemcpyAsync(d_idx, idx, static_cast<size_t>(n_idx) * 4, cudaMemcpyHostToDevice, s));
         launch_fstat_assemble(*ctx, d_f2, P, d_surv, ns, kind, d_idx, n_stat, m, nr, d_x, s);
-        launch_jackknife(*ctx, d_x, d_bl, m, ns, d_est, d_var, s);
+        launch_jackknife(*ctx, d_x, d_bl, bl, m, d_est, d_var, s);
         STPF2_CUDA(cudaMemcpyAsync(est, d_est, static_cast<size_t>(m) * 8, cudaMemcpyDeviceToHost, s));
         STPF2_CUDA(cudaMemcpyAsync(var, d_var, static_cast<size_t>(m) * 8, cudaMemcpyDeviceToHost, s));
         STPF2_CUDA(cudaStreamSynchronize(s));
@@ -2066,7 +2066,7 @@ stp_status stp_f2_jackknife(stp_ctx* ctx, const double* x, const int32_t* block_
         upload(d_b, bs, s);
         d_e.reserve(static_cast<size_t>(m) * 8);
         d_v.reserve(static_cast<size_t>(m) * 8);
-        launch_jackknife(*ctx, d_x.as<double>(), d_b.as<int32_t>(), m, n_block, d_e.as<double>(), d_v.as<double>(), s);
+        launch_jackknife(*ctx, d_x.as<double>(), d_b.as<int32_t>(), bs, m, d_e.as<double>(), d_v.as<double>(), s);
         STPF2_CUDA(cudaMemcpyAsync(est, d_e.ptr, static_cast<size_t>(m) * 8, cudaMemcpyDeviceToHost, s));
         STPF2_CUDA(cudaMemcpyAsync(var, d_v.ptr, static_cast<size_t>(m) * 8, cudaMemcpyDeviceToHost, s));
         STPF2_CUDA(cudaStreamSynchronize(s));

@@ -458,8 +458,9 @@ int umma_tile();
 void launch_survivors(Ctx& c, const double* vpair, int P, int nb, int32_t* keep, cudaStream_t s);
 void launch_fstat_assemble(Ctx& c, const double* f2, int P, const int32_t* surv, int ns, int kind,
                            const int32_t* idx, int64_t n_stat, int64_t m, int64_t nr, double* x, cudaStream_t s);
-void launch_jackknife(Ctx& c, const double* x, const int32_t* block_sizes, int64_t m, int nb,
-                      double* est, double* var, cudaStream_t s);
+// block_sizes: the device copy of sizes.
+void launch_jackknife(Ctx& c, const double* x, const int32_t* block_sizes, const std::vector<int32_t>& sizes,
+                      int64_t m, double* est, double* var, cudaStream_t s);
 
 // Host-output transfer (counts_pack.cu, host_expand.cpp): the upper 128 x 128 tiles of nb
 // count slabs packed as 16-bit (wide: 32-bit) integers, and their widening on the host into

@@ -251,12 +251,37 @@ __device__ __forceinline__ void bytes4x4(uint32_t w0, uint32_t w1, uint32_t w2, 
 }
 
 
+// Where one population's columns from col lie in its fixed-point image: the
+// first of its digit planes, the planes' distance, the plane of -A's digit d and the M tile.
+template <OpFmt F>
+struct FxPlace {
+    uint8_t *img, *m;
+    int plane;
+    __device__ __forceinline__ FxPlace(const OperandPlanes& op, int i, int64_t col) {
+        const int k = static_cast<int>(col % kTileK);
+        if constexpr (F == OpFmt::FXS) {
+            plane = op.small_rows * kTileK;
+            img = static_cast<uint8_t*>(op.planes) + col / kTileK * (kFxsPlanes * plane) + tile8_offset(i, k);
+            m = img + 5 * plane;
+        } else {
+            const int r = i % kTileRows;
+            const int64_t tile = static_cast<int64_t>(i / kTileRows) * op.n_ck + col / kTileK;
+            plane = static_cast<int>(kTile8Bytes);
+            img = static_cast<uint8_t*>(op.planes) + tile * kFxImageBytes + tile8_offset(r, k);
+            m = op.mplanes + tile * kTile8Bytes + tile8_offset(r, k);
+        }
+    }
+    // E_3..E_6 follow X; the stacked order is E_6 M E_3 E_4 E_5.
+    static __device__ __forceinline__ constexpr int e_plane(int d) {
+        return F == OpFmt::FXS ? (d == 3 ? 4 : 6 + d) : 4 + d;
+    }
+};
+
 // Writes 8 consecutive columns (starting at a multiple of 8) of one population into its
-// fixed-point operand image (nine int8 tiles, 8 bytes each) and into the separate M tiles.
+// fixed-point operand image (eight digit planes, 8 bytes each) and its M plane.
+template <OpFmt F>
 __device__ __forceinline__ void emit8_fx(const OperandPlanes& op, int i, int64_t col, const FxTerms8& t) {
-    const int r = i % kTileRows, k = static_cast<int>(col % kTileK);
-    const int64_t tile = static_cast<int64_t>(i / kTileRows) * op.n_ck + col / kTileK;
-    uint8_t* img = static_cast<uint8_t*>(op.planes) + tile * kFxImageBytes + tile8_offset(r, k);
+    const FxPlace<F> at(op, i, col);
     // Digit d of the 8 columns, per plane: two 4 x 4 byte transposes per digit word set.
     uint32_t x0[4], x1[4], n0[4], n1[4];
     bytes4x4(t.x[0], t.x[1], t.x[2], t.x[3], x0);
@@ -265,17 +290,18 @@ __device__ __forceinline__ void emit8_fx(const OperandPlanes& op, int i, int64_t
     bytes4x4(t.na[4], t.na[5], t.na[6], t.na[7], n1);
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
-        *reinterpret_cast<uint2*>(img + d * kTile8Bytes) = make_uint2(x0[d], x1[d]);
-        *reinterpret_cast<uint2*>(img + (4 + d) * kTile8Bytes) = make_uint2(n0[d], n1[d]);
+        *reinterpret_cast<uint2*>(at.img + d * at.plane) = make_uint2(x0[d], x1[d]);
+        *reinterpret_cast<uint2*>(at.img + at.e_plane(d) * at.plane) = make_uint2(n0[d], n1[d]);
     }
     // M = 64 in byte c where column c is called: bit c of each nibble spread to bit 8c.
     static_assert(kFxM == 64, "M is 1 << 6");
     const uint32_t lo = t.mbits & 0xFu, hi = (t.mbits >> 4) & 0xFu;
     const uint2 mv = make_uint2(((lo * 0x00204081u) & 0x01010101u) << 6, ((hi * 0x00204081u) & 0x01010101u) << 6);
-    *reinterpret_cast<uint2*>(op.mplanes + tile * kTile8Bytes + tile8_offset(r, k)) = mv;
+    *reinterpret_cast<uint2*>(at.m) = mv;
 }
 
 // One element (the Q/V/N feeder): q, n as FP64.
+template <OpFmt F>
 __device__ __forceinline__ void emit_fx(const OperandPlanes& op, int i, int64_t col, double q, double nd, bool valid) {
     uint32_t X = 0, NA = 0;
     if (valid) {
@@ -283,16 +309,14 @@ __device__ __forceinline__ void emit_fx(const OperandPlanes& op, int i, int64_t 
         fx_terms(q, 1.0 / ((nm1 > 1.0) ? nm1 : 1.0), X, NA);
     }
     const uint32_t dx = fx_digits(X), dn = fx_digits(NA);
-    const int r = i % kTileRows, k = static_cast<int>(col % kTileK);
-    const int64_t tile = static_cast<int64_t>(i / kTileRows) * op.n_ck + col / kTileK;
-    uint8_t* img = static_cast<uint8_t*>(op.planes) + tile * kFxImageBytes + tile8_offset(r, k);
+    const FxPlace<F> at(op, i, col);
+    uint8_t* img = at.img;
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
-        img[d * kTile8Bytes] = static_cast<uint8_t>(dx >> (8 * d));
-        img[(4 + d) * kTile8Bytes] = static_cast<uint8_t>(dn >> (8 * d));
+        img[d * at.plane] = static_cast<uint8_t>(dx >> (8 * d));
+        img[at.e_plane(d) * at.plane] = static_cast<uint8_t>(dn >> (8 * d));
     }
-    const uint8_t m = valid ? uint8_t(kFxM) : uint8_t(0);
-    op.mplanes[tile * kTile8Bytes + tile8_offset(r, k)] = m;
+    at.m[0] = valid ? uint8_t(kFxM) : uint8_t(0);
 }
 
 // ---- canonical genotypes -------------------------------------------------------------------
@@ -653,7 +677,7 @@ decode_canon_kernel(const uint64_t* __restrict__ canon, int64_t n_tiles, int64_t
     __shared__ double s_center[4 * kCenterPitch];
     const int64_t q = blockIdx.x;
     // Only the split and FP32 operands are centred.
-    for (int c = threadIdx.x; F != OpFmt::FX && op.planes && c < 4 * kTileCols; c += blockDim.x) {
+    for (int c = threadIdx.x; !is_fx(F) && op.planes && c < 4 * kTileCols; c += blockDim.x) {
         const int64_t col = q * 4 * kTileCols + c;
         double cv = 0.5;
         if (col < n_tiles * kTileCols) {
@@ -753,8 +777,8 @@ decode_canon_kernel(const uint64_t* __restrict__ canon, int64_t n_tiles, int64_t
         uint32_t v[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) v[c] = cnt[c * kCntCol];
-        if constexpr (F == OpFmt::FX)
-            emit8_fx(op, i, col_base + col0, fx_terms8_from_counts(v, rec_n, rec_nm1, op.fx_table, op.fx_table_ld));
+        if constexpr (is_fx(F))
+            emit8_fx<F>(op, i, col_base + col0, fx_terms8_from_counts(v, rec_n, rec_nm1, op.fx_table, op.fx_table_ld));
         else
             emit8<F>(op, i, col_base + col0, terms8_from_counts(v, cen, rec_n, rec_nm1));
     }
@@ -857,8 +881,8 @@ __global__ void feed_qvn_kernel(const double* __restrict__ Q, const double* __re
     const int i = blockIdx.y * blockDim.y + threadIdx.y;
     if (s >= M || i >= P) return;
     const int64_t o = static_cast<int64_t>(i) + static_cast<int64_t>(P) * s;
-    if constexpr (F == OpFmt::FX)
-        emit_fx(op, i, snp_col[s], Q[o], N[o], V[o] != 0.0);
+    if constexpr (is_fx(F))
+        emit_fx<F>(op, i, snp_col[s], Q[o], N[o], V[o] != 0.0);
     else
         emit<F>(op, i, snp_col[s], make_terms(Q[o], N[o], V[o] != 0.0, center[s]));
 }
@@ -1082,12 +1106,12 @@ emit_counts_kernel(const uint32_t* __restrict__ counts, int64_t cnt_ld, bool vec
             for (int c = 0; c < 8; ++c) v[c] = sc[c] >= 0 ? __ldg(row + sc[c]) : 0u;
         }
         double cen[8];
-        if constexpr (F != OpFmt::FX) {  // the fixed point needs no centre
+        if constexpr (!is_fx(F)) {  // the fixed point needs no centre
 #pragma unroll
             for (int c = 0; c < 8; ++c) cen[c] = sc[c] >= 0 ? __ldg(center_snp + sc[c]) : 0.5;
         }
-        if constexpr (F == OpFmt::FX)
-            emit8_fx(op, i, col0, fx_terms8_from_counts(v, rec_n, rec_nm1, op.fx_table, op.fx_table_ld));
+        if constexpr (is_fx(F))
+            emit8_fx<F>(op, i, col0, fx_terms8_from_counts(v, rec_n, rec_nm1, op.fx_table, op.fx_table_ld));
         else
             emit8<F>(op, i, col0, terms8_from_counts(v, cen, rec_n, rec_nm1));
     }
@@ -1185,6 +1209,7 @@ void launch_emit_counts(Ctx& c, const uint32_t* counts, int64_t cnt_ld, int64_t 
         case OpFmt::BF16: emit_counts_kernel<OpFmt::BF16><<<grid, 256, 0, s>>>(counts, cnt_ld, vec, upop, P, n_tiles, col_snp, center_snp, rec_n, rec_nm1, op); break;
         case OpFmt::F16: emit_counts_kernel<OpFmt::F16><<<grid, 256, 0, s>>>(counts, cnt_ld, vec, upop, P, n_tiles, col_snp, center_snp, rec_n, rec_nm1, op); break;
         case OpFmt::FX: emit_counts_kernel<OpFmt::FX><<<grid, 256, 0, s>>>(counts, cnt_ld, vec, upop, P, n_tiles, col_snp, center_snp, rec_n, rec_nm1, op); break;
+        case OpFmt::FXS: emit_counts_kernel<OpFmt::FXS><<<grid, 256, 0, s>>>(counts, cnt_ld, vec, upop, P, n_tiles, col_snp, center_snp, rec_n, rec_nm1, op); break;
     }
     STPF2_CUDA(cudaGetLastError());
     c.launches++;
@@ -1206,13 +1231,14 @@ void launch_decode_canon(Ctx& c, const CanonDecodeArgs& a, cudaStream_t s) {
 #define STPF2_DECODE_LAUNCH(F)                                                                      \
     (a.umap ? decode_canon_kernel<F, true><<<grid, kDecThreads2, kDecSmemBytes, s>>>(STPF2_DECODE_ARGS) \
             : decode_canon_kernel<F, false><<<grid, kDecThreads2, kDecSmemBytes, s>>>(STPF2_DECODE_ARGS))
-    if (a.op.fmt != OpFmt::FX && a.op.planes && !(a.umap ? a.center_snp : a.center))
+    if (!is_fx(a.op.fmt) && a.op.planes && !(a.umap ? a.center_snp : a.center))
         fail(STP_INVALID_ARGUMENT, "decode of centred operands needs the centres");
     switch (a.op.fmt) {
         case OpFmt::F32: STPF2_DECODE_LAUNCH(OpFmt::F32); break;
         case OpFmt::BF16: STPF2_DECODE_LAUNCH(OpFmt::BF16); break;
         case OpFmt::F16: STPF2_DECODE_LAUNCH(OpFmt::F16); break;
         case OpFmt::FX: STPF2_DECODE_LAUNCH(OpFmt::FX); break;
+        case OpFmt::FXS: STPF2_DECODE_LAUNCH(OpFmt::FXS); break;
     }
 #undef STPF2_DECODE_LAUNCH
 #undef STPF2_DECODE_ARGS
@@ -1256,6 +1282,7 @@ void launch_feed_qvn(Ctx& c, const double* Q, const double* V, const double* N, 
         case OpFmt::BF16: feed_qvn_kernel<OpFmt::BF16><<<grid, block, 0, s>>>(Q, V, N, P, M, snp_col, center, op); break;
         case OpFmt::F16: feed_qvn_kernel<OpFmt::F16><<<grid, block, 0, s>>>(Q, V, N, P, M, snp_col, center, op); break;
         case OpFmt::FX: feed_qvn_kernel<OpFmt::FX><<<grid, block, 0, s>>>(Q, V, N, P, M, snp_col, center, op); break;
+        case OpFmt::FXS: feed_qvn_kernel<OpFmt::FXS><<<grid, block, 0, s>>>(Q, V, N, P, M, snp_col, center, op); break;
     }
     STPF2_CUDA(cudaGetLastError());
     c.launches++;

@@ -355,17 +355,6 @@ __device__ __forceinline__ void stamp(const FxArgs& a, int grp, int lane) {
     }
 }
 
-// int64 -> FP64 without a conversion instruction: each 32-bit half is placed in the
-// mantissa of 2^52 (2^52 + 2^31 for the signed high half) by its bit pattern and the bias
-// subtracted exactly; hi * 2^32 + lo then rounds once (a correctly rounded conversion).
-__device__ __forceinline__ double i64_to_f64(int64_t w) {
-    const int lo = static_cast<int>(static_cast<uint32_t>(w));
-    const int hi = static_cast<int>(static_cast<uint32_t>(static_cast<uint64_t>(w) >> 32) ^ 0x80000000u);
-    const double dl = __hiloint2double(0x43300000, lo) - 4503599627370496.0;  // 2^52
-    const double dh = __hiloint2double(0x43300000, hi) - 4503601774854144.0;  // 2^52 + 2^31
-    return fma(dh, 4294967296.0, dl);
-}
-
 __device__ __forceinline__ void st_cs_v2(double* p, double x, double y) {
     asm volatile("st.global.cs.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(x), "d"(y) : "memory");
 }

@@ -531,6 +531,7 @@ struct UmmaPlan {
     DevBuf items, blocks, err, rcp, block_items, counter;
     DevBuf vpc;  // FX: compact vpair tiles, one per item of the largest launch
     DevBuf units, block_units;  // FX: vpair units of items and of block_items
+    DevBuf work, block_work;    // FXS: one item per block, costliest first and in block order
     std::vector<int> block_item_off;  // per block: its tile pairs in block_items
     std::vector<int> block_unit_off;  // per block: its vpair units in block_units
     int n_items = 0;
@@ -544,6 +545,40 @@ struct UmmaPlan {
 
 int umma_tile() { return kTile; }
 
+namespace {
+
+// Reciprocals of every count a block can reach, 1/0 as 0.
+std::vector<double> reciprocals(int max_k) {
+    std::vector<double> rcp(static_cast<size_t>(max_k) + 1, 0.0);
+    for (int k = 1; k <= max_k; ++k) rcp[k] = 1.0 / static_cast<double>(k);
+    return rcp;
+}
+
+int longest_block(const BlockLayout& L) {
+    int k = 0;
+    for (const BlockInfo& b : L.blocks) k = std::max(k, b.k);
+    return k;
+}
+
+std::vector<BlockInfo> costliest_first(const BlockLayout& L) {
+    std::vector<BlockInfo> w(L.blocks);
+    std::stable_sort(w.begin(), w.end(), [](const BlockInfo& x, const BlockInfo& y) { return x.k > y.k; });
+    return w;
+}
+
+// A plan's reciprocals, cleared error flag and work counter.
+void upload_control(Ctx& c, UmmaPlan& p, const BlockLayout& L) {
+    p.err.reserve(16);
+    p.counter.reserve(16);
+    STPF2_CUDA(cudaMemsetAsync(p.err.ptr, 0, 16, c.stream));
+    const std::vector<double> rcp = reciprocals(p.rcp_max = longest_block(L));
+    p.rcp.reserve(rcp.size() * sizeof(double));
+    STPF2_CUDA(cudaMemcpyAsync(p.rcp.ptr, rcp.data(), rcp.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    STPF2_CUDA(cudaStreamSynchronize(c.stream));
+}
+
+}  // namespace
+
 UmmaPlan* umma_plan_create(Ctx& c, const OperandPlanes& op, const BlockLayout& L, int chunk_stages) {
     if (op.fmt == OpFmt::F32) fail(STP_INVALID_ARGUMENT, "tensor-core contraction needs tiled operand images");
     auto p = std::make_unique<UmmaPlan>();
@@ -552,6 +587,20 @@ UmmaPlan* umma_plan_create(Ctx& c, const OperandPlanes& op, const BlockLayout& L
     p->fmt = op.fmt;
     p->chunk_stages = chunk_stages;
     p->num_scale = 2.0 * op.scale_inv;
+    if (op.fmt == OpFmt::FXS) {
+        p->n_items = static_cast<int>(L.blocks.size());
+        p->images = static_cast<const uint8_t*>(op.planes);
+        const std::vector<BlockInfo> work = costliest_first(L);
+        p->work.reserve(std::max<size_t>(work.size() * sizeof(BlockInfo), 16));
+        p->block_work.reserve(std::max<size_t>(work.size() * sizeof(BlockInfo), 16));
+        STPF2_CUDA(cudaMemcpyAsync(p->work.ptr, work.data(), work.size() * sizeof(BlockInfo), cudaMemcpyHostToDevice, c.stream));
+        STPF2_CUDA(cudaMemcpyAsync(p->block_work.ptr, L.blocks.data(), L.blocks.size() * sizeof(BlockInfo),
+                                   cudaMemcpyHostToDevice, c.stream));
+        upload_control(c, *p, L);
+        STPF2_CUDA(cudaStreamSynchronize(c.stream));  // the host tables above go out of scope
+        fxs_prepare();
+        return p.release();
+    }
     const std::vector<WorkItem> items = make_work_items(L, op.P, kTile);
     p->n_items = static_cast<int>(items.size());
     // The same items grouped by block, for the one-launch-per-block comparison form.
@@ -565,20 +614,11 @@ UmmaPlan* umma_plan_create(Ctx& c, const OperandPlanes& op, const BlockLayout& L
                                cudaMemcpyHostToDevice, c.stream));
     p->items.reserve(std::max<size_t>(items.size() * sizeof(WorkItem), 16));
     p->blocks.reserve(std::max<size_t>(L.blocks.size() * sizeof(BlockInfo), 16));
-    p->err.reserve(16);
-    p->counter.reserve(16);
     STPF2_CUDA(cudaMemcpyAsync(p->items.ptr, items.data(), items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice,
                                c.stream));
     STPF2_CUDA(cudaMemcpyAsync(p->blocks.ptr, L.blocks.data(), L.blocks.size() * sizeof(BlockInfo),
                                cudaMemcpyHostToDevice, c.stream));
-    STPF2_CUDA(cudaMemsetAsync(p->err.ptr, 0, 16, c.stream));
-    int max_k = 0;
-    for (const BlockInfo& b : L.blocks) max_k = std::max(max_k, b.k);
-    std::vector<double> rcp(static_cast<size_t>(max_k) + 1, 0.0);
-    for (int k = 1; k <= max_k; ++k) rcp[k] = 1.0 / static_cast<double>(k);
-    p->rcp_max = max_k;
-    p->rcp.reserve(rcp.size() * sizeof(double));
-    STPF2_CUDA(cudaMemcpyAsync(p->rcp.ptr, rcp.data(), rcp.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    upload_control(c, *p, L);
     std::vector<int32_t> units, block_units;
     if (op.fmt == OpFmt::FX) {
         units = make_vpair_units(items);
@@ -615,8 +655,27 @@ void umma_plan_destroy(UmmaPlan* p) { delete p; }
 void launch_umma_items(Ctx& c, UmmaPlan* p, const WorkItem* items, int n_items, double* f2, double* vpair,
                        cudaStream_t s, int b_base = 0, int b0 = -1, int b1 = -1);
 
+// n items of an FXS work list.
+void launch_fxs_items(Ctx& c, UmmaPlan* p, const BlockInfo* work, int n, double* f2, double* vpair, cudaStream_t s,
+                      int b_base) {
+    FxsLaunch L;
+    L.images = p->images;
+    L.work = work;
+    L.n_work = n;
+    L.P = p->P;
+    L.f2 = f2;
+    L.vpair = vpair;
+    L.rcp = p->rcp.as<double>();
+    L.rcp_max = p->rcp_max;
+    L.err = p->err.as<int>();
+    L.counter = p->counter.as<int>();
+    L.b_base = b_base;
+    launch_fxs(c, L, s);
+}
+
 void launch_f2_umma(Ctx& c, UmmaPlan* p, double* f2, double* vpair, cudaStream_t s, bool per_block) {
     if (!p || p->n_items <= 0) return;
+    if (p->fmt == OpFmt::FXS) return launch_fxs_items(c, p, p->work.as<BlockInfo>(), p->n_items, f2, vpair, s, 0);
     if (per_block) {  // comparison form: one launch per jackknife block
         for (size_t b = 0; b + 1 < p->block_item_off.size(); ++b) {
             const int n = p->block_item_off[b + 1] - p->block_item_off[b];
@@ -632,6 +691,8 @@ void launch_f2_umma(Ctx& c, UmmaPlan* p, double* f2, double* vpair, cudaStream_t
 void launch_f2_umma_blocks(Ctx& c, UmmaPlan* p, int b0, int b1, double* f2, double* vpair, cudaStream_t s,
                            bool rebase) {
     if (!p || b1 <= b0) return;
+    if (p->fmt == OpFmt::FXS)
+        return launch_fxs_items(c, p, p->block_work.as<BlockInfo>() + b0, b1 - b0, f2, vpair, s, rebase ? b0 : 0);
     const int n = p->block_item_off[static_cast<size_t>(b1)] - p->block_item_off[static_cast<size_t>(b0)];
     if (n > 0)
         launch_umma_items(c, p, p->block_items.as<WorkItem>() + p->block_item_off[static_cast<size_t>(b0)], n, f2, vpair, s,
@@ -706,8 +767,11 @@ void launch_umma_items(Ctx& c, UmmaPlan* p, const WorkItem* items, int n_items, 
     c.launches++;
 }
 
-void launch_f2_umma_grouped(Ctx& c, OpFmt fmt, double scale_inv, int chunk_stages, const std::vector<GroupSpec>& groups,
+void launch_f2_umma_grouped(Ctx& c, double scale_inv, int chunk_stages, const std::vector<GroupSpec>& groups,
                             cudaStream_t s, std::vector<unsigned long long>* stamps) {
+    OpFmt fmt = OpFmt::FXS;  // the format of the requests that are not FXS
+    for (const GroupSpec& g : groups)
+        if (g.fmt != OpFmt::FXS) fmt = g.fmt;
     if (fmt == OpFmt::F32) fail(STP_INVALID_ARGUMENT, "tensor-core contraction needs tiled operand images");
     if (chunk_stages != 1 && chunk_stages != 2) fail(STP_INVALID_ARGUMENT, "chunk stages must be 1 or 2");
     const int G = static_cast<int>(groups.size());
@@ -724,12 +788,23 @@ void launch_f2_umma_grouped(Ctx& c, OpFmt fmt, double scale_inv, int chunk_stage
     std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return cost[x] < cost[y]; });
     std::vector<BlockInfo> blocks;
     std::vector<WorkItem> items;
+    std::vector<BlockInfo> work;  // the FXS requests' items
     std::vector<int> n_items(static_cast<size_t>(G), 0);
     std::vector<GroupInfo> info(static_cast<size_t>(G));
     int max_k = 0;
     for (int g : ord) {
         const BlockLayout& L = *groups[g].L;
         info[g] = groups[g].info;
+        if (groups[g].fmt == OpFmt::FXS) {
+            for (BlockInfo b : costliest_first(L)) {
+                b.grp = g;
+                b.P = info[g].P;
+                work.push_back(b);
+                max_k = std::max(max_k, b.k);
+            }
+            n_items[g] = L.n_block;
+            continue;
+        }
         const int base = static_cast<int>(blocks.size());
         for (BlockInfo b : L.blocks) {
             b.grp = g;
@@ -743,10 +818,9 @@ void launch_f2_umma_grouped(Ctx& c, OpFmt fmt, double scale_inv, int chunk_stage
             n_items[g]++;
         }
     }
-    if (items.empty()) return;
-    if (items.size() > static_cast<size_t>(INT_MAX)) fail(STP_RUNTIME_ERROR, "too many work items in one batch");
-    std::vector<double> rcp(static_cast<size_t>(max_k) + 1, 0.0);
-    for (int k = 1; k <= max_k; ++k) rcp[k] = 1.0 / static_cast<double>(k);
+    if (items.empty() && work.empty()) return;
+    if (std::max(items.size(), work.size()) > static_cast<size_t>(INT_MAX)) fail(STP_RUNTIME_ERROR, "too many work items in one batch");
+    const std::vector<double> rcp = reciprocals(max_k);
     // Every table in one pinned staging buffer and one upload; counters cleared on device.
     Packing pk;
     const size_t o_items = pk.add(items.size() * sizeof(WorkItem));
@@ -757,11 +831,13 @@ void launch_f2_umma_grouped(Ctx& c, OpFmt fmt, double scale_inv, int chunk_stage
     const bool fx = fmt == OpFmt::FX;
     const std::vector<int32_t> units = fx ? make_vpair_units(items) : std::vector<int32_t>();
     const size_t o_units = pk.add(units.size() * sizeof(int32_t));
+    const size_t o_work = pk.add(work.size() * sizeof(BlockInfo));
     const size_t staged = pk.end;
     const size_t o_done = pk.add(static_cast<size_t>(G) * sizeof(int));
     const size_t o_ns = pk.add(static_cast<size_t>(G) * sizeof(unsigned long long));
     const size_t o_err = pk.add(16);
     const size_t o_counter = pk.add(16);
+    const size_t o_counter_s = pk.add(16);
     if (fx) c.ws_vpc.reserve(fx_vpc_bytes(static_cast<int>(items.size())));
     c.pin_items.reserve(staged);
     c.ws_items.reserve(pk.end);
@@ -771,11 +847,28 @@ void launch_f2_umma_grouped(Ctx& c, OpFmt fmt, double scale_inv, int chunk_stage
     std::memcpy(h + o_info, info.data(), info.size() * sizeof(GroupInfo));
     std::memcpy(h + o_rcp, rcp.data(), rcp.size() * sizeof(double));
     std::memcpy(h + o_nitems, n_items.data(), n_items.size() * sizeof(int));
+    if (!work.empty()) std::memcpy(h + o_work, work.data(), work.size() * sizeof(BlockInfo));
     if (!units.empty()) std::memcpy(h + o_units, units.data(), units.size() * sizeof(int32_t));
     uint8_t* d = c.ws_items.as<uint8_t>();
     STPF2_CUDA(cudaMemcpyAsync(d, h, staged, cudaMemcpyHostToDevice, s));
     STPF2_CUDA(cudaMemsetAsync(d + staged, 0, pk.end - staged, s));
-    if (fx) {
+    if (!work.empty()) {
+        fxs_prepare();
+        FxsLaunch L;
+        L.work = reinterpret_cast<const BlockInfo*>(d + o_work);
+        L.n_work = static_cast<int>(work.size());
+        L.rcp = reinterpret_cast<const double*>(d + o_rcp);
+        L.rcp_max = max_k;
+        L.err = reinterpret_cast<int*>(d + o_err);
+        L.counter = reinterpret_cast<int*>(d + o_counter_s);
+        L.groups = reinterpret_cast<const GroupInfo*>(d + o_info);
+        L.grp_done = reinterpret_cast<int*>(d + o_done);
+        L.grp_ns = reinterpret_cast<unsigned long long*>(d + o_ns);
+        L.grp_items = reinterpret_cast<const int*>(d + o_nitems);
+        launch_fxs(c, L, s);
+    }
+    if (items.empty()) {
+    } else if (fx) {
         fx_prepare();
         FxLaunch L;
         L.images = info[ord[0]].images;

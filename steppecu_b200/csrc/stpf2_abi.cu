@@ -138,6 +138,7 @@ size_t operand_plane_bytes(OpFmt f, int P, int64_t ld) {
         const size_t pl = static_cast<size_t>(P) * static_cast<size_t>(ld);
         return align256(2 * pl * 4) + align256(pl);
     }
+    if (f == OpFmt::FXS) return align256(static_cast<size_t>(ld / kTileK) * kFxsPlanes * kTileK * fxs_rows(P));
     const size_t tiles = static_cast<size_t>((P + kTileRows - 1) / kTileRows) * static_cast<size_t>(ld / kTileK);
     if (f == OpFmt::FX) return align256(tiles * (kFxImageBytes + kTile8Bytes));  // images, then the M tiles
     return align256(tiles * kImageBytes);
@@ -157,6 +158,7 @@ void bind_operand_planes(OperandPlanes& op, OpFmt f, int P, int64_t ld, void* ba
     } else {
         op.n_rt = (P + kTileRows - 1) / kTileRows;
         op.n_ck = ld / kTileK;
+        op.small_rows = f == OpFmt::FXS ? fxs_rows(P) : 0;
         op.m_u8 = nullptr;  // the int8 M tiles live inside the operand images (FX: after them)
         op.mplanes = f == OpFmt::FX ? static_cast<uint8_t*>(base) + static_cast<size_t>(op.n_rt) * op.n_ck * kFxImageBytes
                                     : nullptr;
@@ -207,12 +209,28 @@ struct Plan {
 
     int launches() const {
         int contract = (per_block && umma) ? static_cast<int>(L.blocks.size()) : 1;
-        if (precision == STP_PREC_FIXED_I8) contract *= 2;  // the vpair kernel, then the f2 kernel
+        if (op.fmt == OpFmt::FX) contract *= 2;  // the vpair kernel, then the f2 kernel
         return (detect ? 1 : 0) + 2 + contract;
     }
 };
 
 namespace {
+
+// Operand planes of one format (at planes_base, or the plan's own) and the tensor-core plan
+// that reads them. Padding columns must read as zero; decode only ever writes real SNP columns.
+void bind_contraction(Plan& p, OpFmt fmt, void* planes_base) {
+    const size_t ob = operand_plane_bytes(fmt, std::max(p.P, 1), p.L.ld);
+    if (!planes_base) {
+        p.own_planes.reserve(ob);
+        planes_base = p.own_planes.ptr;
+    }
+    STPF2_CUDA(cudaMemsetAsync(planes_base, 0, ob, p.ctx->stream));
+    bind_operand_planes(p.op, fmt, p.P, p.L.ld, planes_base);
+    if (p.umma) umma_plan_destroy(p.umma);
+    p.umma = nullptr;
+    if (fmt != OpFmt::F32 && p.P > 0 && p.L.n_block > 0)
+        p.umma = umma_plan_create(*p.ctx, p.op, p.L, chunk_stages_of(p.precision));
+}
 
 // Validates a request and builds its plan. planes_base != nullptr borrows operand
 // storage (at least operand_plane_bytes) instead of allocating it; borrow_ws takes the
@@ -243,7 +261,7 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     }
     p->pitch = pitch;
     p->precision = r.precision;
-    const OpFmt fmt = fmt_of(r.precision);
+    fmt_of(r.precision);  // validates the mode
     const int64_t n_sel = r.n_pop > 0 ? r.pop_offsets[r.n_pop] : 0;
     p->n_sel = n_sel;
     need(r.n_pop == 0 || r.pop_offsets[0] == 0, "pop_offsets[0] must be 0");
@@ -355,30 +373,21 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     upload(p->blocks, p->L.blocks, s);
     if (counts_only) return p;  // decode to counts only: no operand planes, no contraction
 
-    const size_t ob = operand_plane_bytes(fmt, std::max(r.n_pop, 1), p->L.ld);
-    if (!planes_base) {
-        p->own_planes.reserve(ob);
-        planes_base = p->own_planes.ptr;
-    }
-    // Padding columns must read as zero; decode only ever writes real SNP columns. A plan
-    // cached on the context relies on that for the shared planes workspace, so building
-    // another plan there drops it.
-    if (planes_base == c.ws_misc.ptr) c.plan_cache.reset();
-    STPF2_CUDA(cudaMemsetAsync(planes_base, 0, ob, s));
-    bind_operand_planes(p->op, fmt, r.n_pop, p->L.ld, planes_base);
-    if (fmt == OpFmt::FX && fx_table_entries(n_max) > 0) {
+    // A plan cached on the context borrows the shared planes workspace, so building another
+    // plan there drops it.
+    if (planes_base && planes_base == c.ws_misc.ptr) c.plan_cache.reset();
+    const OpFmt fmt = operand_fmt(r.precision, r.n_pop, p->L);
+    if (is_fx(fmt) && fx_table_entries(n_max) > 0) {
         p->fx_table.reserve(static_cast<size_t>(fx_table_entries(n_max)) * sizeof(uint2));
         launch_fx_table(c, p->rec_n.as<double>(), p->rec_nm1.as<double>(), n_max, p->fx_table.as<uint2>(), s);
         p->op.fx_table = p->fx_table.as<uint2>();
         p->op.fx_table_ld = static_cast<int32_t>(2 * n_max + 1);
     }
-
+    bind_contraction(*p, fmt, planes_base);
     if (r.precision == STP_PREC_FP32_SIMT) {
         const std::vector<WorkItem> items = make_work_items(p->L, r.n_pop, simt_tile());
         p->n_items = static_cast<int>(items.size());
         upload(p->items, items, s);
-    } else if (r.n_pop > 0 && r.n_block > 0) {
-        p->umma = umma_plan_create(c, p->op, p->L, chunk_stages_of(r.precision));
     }
     return p;
 }
@@ -400,7 +409,7 @@ void launch_decode(Plan& p, const uint8_t* d_records, int32_t* cnt_ac2, int32_t*
         launch_detect_ploidy_words(c, rec, p.pitch, p.bpr, p.n_rec, p.n_ind, p.pos.as<int32_t>(), p.sel.as<uint32_t>(), s);
     if (t1 <= t0) return;
     const bool counts = cnt_ac2 || cnt_packed;
-    double* center = p.op.fmt == OpFmt::FX || counts ? nullptr : p.center_ptr + t0 * kTileK;
+    double* center = is_fx(p.op.fmt) || counts ? nullptr : p.center_ptr + t0 * kTileK;
     launch_transpose_pa(c, rec, p.pitch, p.bpr, p.n_ind, p.tiles.as<TileInfo>() + t0, t1 - t0, p.pos.as<int32_t>(),
                         p.n_sel_pad, p.canon_ptr, center, s, p.row_map.as<int32_t>());
     CanonDecodeArgs a;
@@ -885,7 +894,7 @@ void extract_one(Ctx& c, const stp_f2_request& r, stp_f2_output& o) {
     const bool hit = p != nullptr;
     if (!hit) {
         const BlockLayout probe = make_block_layout(r.block_id, snp_axis(r), r.n_block);
-        c.ws_misc.reserve(operand_plane_bytes(fmt_of(r.precision), std::max(r.n_pop, 1), probe.ld));
+        c.ws_misc.reserve(operand_plane_bytes(operand_fmt(r.precision, r.n_pop, probe), std::max(r.n_pop, 1), probe.ld));
         p = build_plan(c, r, pitch, c.ws_misc.ptr, true);
     }
     if (o.block_sizes) copy_block_sizes(p->L, o.block_sizes);
@@ -945,12 +954,13 @@ struct BatchMember {
     std::vector<int32_t> plcode;             // per selected sample: 0/1/2, or 3 = detect
     std::vector<int32_t> upop;               // population -> batch population
     size_t img_bytes = 0, out_bytes = 0, vpc_bytes = 0;
+    OpFmt fmt = OpFmt::BF16;
     OperandPlanes op;
 };
 
 // Validates request r (the rules of build_plan) and fills m's host tables. Host only,
 // safe to run for several members at once.
-void prepare_member(const stp_f2_request& r, const stp_f2_output& o, int64_t n_ind, OpFmt fmt, BatchMember& m) {
+void prepare_member(const stp_f2_request& r, const stp_f2_output& o, int64_t n_ind, BatchMember& m) {
     need(r.n_pop > 0 && r.n_block > 0, "empty request in a batch");
     need(r.pop_offsets != nullptr, "pop_offsets is NULL");
     need(r.pop_offsets[0] == 0, "pop_offsets[0] must be 0");
@@ -988,8 +998,9 @@ void prepare_member(const stp_f2_request& r, const stp_f2_output& o, int64_t n_i
         std::sort(key.begin(), key.end());
     }
     m.L = make_block_layout(r.block_id, r.geno.n_snp, r.n_block, false);
-    m.img_bytes = align256(operand_plane_bytes(fmt, r.n_pop, m.L.ld));
-    if (fmt == OpFmt::FX) {  // the compact vpair tiles of the member's work items (context workspace)
+    m.fmt = operand_fmt(r.precision, r.n_pop, m.L);
+    m.img_bytes = align256(operand_plane_bytes(m.fmt, r.n_pop, m.L.ld));
+    if (m.fmt == OpFmt::FX) {  // the compact vpair tiles of the member's work items (context workspace)
         const int64_t T = (r.n_pop + kTileRows - 1) / kTileRows;
         m.vpc_bytes = fx_vpc_bytes(static_cast<int>(std::min<int64_t>(INT_MAX, r.n_block * T * (T + 1) / 2)));
     }
@@ -1103,7 +1114,7 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
     std::vector<BatchMember> mem(idx.size());
     parallel_for(static_cast<int>(idx.size()), [&](int m) {
         mem[m].k = idx[m];
-        prepare_member(reqs[idx[m]], outs[idx[m]], n_ind, fmt, mem[m]);
+        prepare_member(reqs[idx[m]], outs[idx[m]], n_ind, mem[m]);
     });
 
     // The batch's distinct populations, decoded once into packed counts.
@@ -1255,7 +1266,7 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
             BatchMember& p = mem[wave[w]];
             const MemberOffsets& q = mo[wave[w]];
             const stp_f2_output& o = outs[p.k];
-            bind_operand_planes(p.op, fmt, p.P, p.L.ld, c.ws_batch.as<uint8_t>() + io);
+            bind_operand_planes(p.op, p.fmt, p.P, p.L.ld, c.ws_batch.as<uint8_t>() + io);
             p.op.fx_table = d_fxtab;
             p.op.fx_table_ld = static_cast<int32_t>(2 * n_max + 1);
             io += p.img_bytes;
@@ -1270,12 +1281,13 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
                 oo += p.out_bytes / 2;
             }
             specs[w].L = &p.L;
+            specs[w].fmt = p.fmt;
             specs[w].info = GroupInfo{static_cast<const uint8_t*>(p.op.planes), f2, vp, p.op.n_ck, p.P, 0, p.op.mplanes};
             if (o.block_sizes) copy_block_sizes(p.L, o.block_sizes);
         }
         fork.join();
         std::vector<unsigned long long> stamps;
-        launch_f2_umma_grouped(c, fmt, mem[wave[0]].op.scale_inv, chunk_stages_of(prec), specs, s, &stamps);
+        launch_f2_umma_grouped(c, mem[wave[0]].op.scale_inv, chunk_stages_of(prec), specs, s, &stamps);
         if (t0 == 0) STPF2_CUDA(cudaMemcpy(&t0, d_t0, sizeof(t0), cudaMemcpyDeviceToHost));
         for (size_t w = 0; w < wave.size(); ++w) {
             BatchMember& p = mem[wave[w]];
@@ -1737,8 +1749,7 @@ void f2_from_qvn(Ctx& c, const double* Q, const double* V, const double* N, int 
     if (n_block > 0 && block_sizes) std::fill(block_sizes, block_sizes + n_block, 0);
     if (P <= 0 || n_block <= 0) return;
     cudaStream_t s = c.stream;
-    const OpFmt fmt = fmt_of(precision);
-    if (t.sink) need(fmt != OpFmt::F32, "streamed output needs a tensor-core precision");
+    if (t.sink) need(fmt_of(precision) != OpFmt::F32, "streamed output needs a tensor-core precision");
     else need(t.f2 && t.vpair, "null output");
     if (M <= 0) {  // every block is empty: zeros (cpu_backend.cpp:234)
         if (t.sink) {
@@ -1757,6 +1768,7 @@ void f2_from_qvn(Ctx& c, const double* Q, const double* V, const double* N, int 
     need(Q && V && N && block_id, "null input");
     DrainOnError drain{c};
     const BlockLayout L = make_block_layout(block_id, M, n_block);
+    const OpFmt fmt = operand_fmt(precision, P, L);
     if (block_sizes) copy_block_sizes(L, block_sizes);
     DevBuf d_qvn, d_col, d_planes, d_blocks, d_items, d_f2, d_vp;
     const size_t pm = static_cast<size_t>(P) * M;
@@ -1875,7 +1887,7 @@ stp_status stp_f2_extract_streamed(stp_ctx* ctx, const stp_f2_request* req, stp_
         }
         {
             const BlockLayout probe = make_block_layout(r.block_id, snp_axis(r), r.n_block);
-            c.ws_misc.reserve(operand_plane_bytes(fmt_of(r.precision), std::max(r.n_pop, 1), probe.ld));
+            c.ws_misc.reserve(operand_plane_bytes(operand_fmt(r.precision, r.n_pop, probe), std::max(r.n_pop, 1), probe.ld));
         }
         std::unique_ptr<Plan> p = build_plan(c, r, dp, c.ws_misc.ptr, true);
         need(p->words || !r.geno.on_device, "streamed extraction of device records needs a 4-byte aligned pitch");
@@ -2142,7 +2154,17 @@ int32_t stp_plan_launches(const stp_plan* plan) { return plan ? plan->p->launche
 stp_status stp_plan_set_per_block_launch(stp_plan* plan, int32_t enable) {
     return guarded([&] {
         need(plan != nullptr, "null plan");
-        plan->p->per_block = enable != 0;
+        Plan& p = *plan->p;
+        use_device(*p.ctx);
+        // The comparison form runs the general kernels: up to kFxsMaxPops populations the
+        // plan's operands change between the stacked layout and the general one.
+        const OpFmt fmt = enable ? fmt_of(p.precision) : operand_fmt(p.precision, p.P, p.L);
+        if (p.umma && fmt != p.op.fmt) {
+            STPF2_CUDA(cudaDeviceSynchronize());  // runs on any stream still read the operands
+            bind_contraction(p, fmt, nullptr);
+            STPF2_CUDA(cudaStreamSynchronize(p.ctx->stream));
+        }
+        p.per_block = enable != 0;
         if (plan->p->graph) {  // the captured graph holds the other launch form
             STPF2_CUDA(cudaGraphExecDestroy(plan->p->graph));
             plan->p->graph = nullptr;

@@ -156,12 +156,12 @@ struct BlockInfo {  // device-visible, one per jackknife block
     int32_t k;        // SNPs in the block
     int32_t b;        // block id (slab index of the output)
     int32_t grp = 0;  // request of a batch (index into the GroupInfo table)
-    int32_t pad_ = 0;
+    int32_t P = 0;    // FXS batches: the request's populations
 };
 
 // One request of a grouped contraction: its operand images and its output slabs.
 struct GroupInfo {
-    const uint8_t* images;  // (row tile t, chunk c) at (t * n_ck + c) * kImageBytes (FX: kFxImageBytes)
+    const uint8_t* images;  // (row tile t, chunk c) at (t * n_ck + c) * kImageBytes (FX: kFxImageBytes; FXS: its own)
     double* f2;             // [P x P x n_block]
     double* vpair;
     int64_t n_ck;
@@ -205,7 +205,10 @@ std::vector<int32_t> make_vpair_units(const std::vector<WorkItem>& items);
 // ---- operand planes --------------------------------------------------------------------
 
 // Operand formats the decode/feeder kernels emit, one per contraction arithmetic.
-enum class OpFmt : int { F32 = 0, BF16 = 1, F16 = 2, FX = 3 };
+// FXS is FX's layout for at most kFxsMaxPops populations.
+enum class OpFmt : int { F32 = 0, BF16 = 1, F16 = 2, FX = 3, FXS = 4 };
+
+constexpr bool is_fx(OpFmt f) { return f == OpFmt::FX || f == OpFmt::FXS; }
 
 inline OpFmt fmt_of(int precision) {
     switch (precision) {
@@ -245,6 +248,7 @@ struct OperandPlanes {
     const uint2* fx_table = nullptr;
     int32_t fx_table_ld = 0;
     double scale_inv = 1.0;  // numerator scale undo (F16 planes are pre-scaled)
+    int small_rows = 0;      // FXS: rows per plane
     int n_rt = 0;            // tiled: row tiles of 128 populations
     int64_t n_ck = 0;        // tiled: column chunks of 32
 };
@@ -284,6 +288,35 @@ constexpr int kFxM = 64;
 // f2 numerator from W = sum_w V_w 2^(8(w-3)) (the four int32 accumulators): num = -2^25 W /
 // kFxScale^2 = -W / (16129 * 2^25).
 constexpr double kFxNumScale = -1.0 / (16129.0 * 33554432.0);
+
+// FXS (f2_fxs.cu): one image per chunk of nine planes [X0 X1 X2 X3 E6 M E3 E4 E5] of R =
+// fxs_rows(P) rows x 32 bytes (the same digits and swizzle), chunk c at c * kFxsPlanes * 32 * R.
+// The order puts every operand of the two MMAs of a chunk on consecutive planes.
+constexpr int kFxsPlanes = 9;
+constexpr int kFxsMaxPops = 64;            // 4R MMA columns and 2 x 4R accumulator columns at most
+constexpr int32_t kFxsMaxBlock = 1 << 22;  // SNPs of a block whose sums stay below 2^63
+__host__ __device__ inline int fxs_rows(int P) { return (P + 7) / 8 * 8; }
+// The operand format of a request: the stacked planes where they hold it, else its mode's own.
+inline OpFmt operand_fmt(int precision, int P, const BlockLayout& L) {
+    const OpFmt f = fmt_of(precision);
+    if (f != OpFmt::FX || P > kFxsMaxPops) return f;
+    for (const BlockInfo& b : L.blocks)
+        if (b.k > kFxsMaxBlock) return f;
+    return OpFmt::FXS;
+}
+
+#ifdef __CUDACC__
+// int64 -> FP64 without a conversion instruction: each 32-bit half is placed in the
+// mantissa of 2^52 (2^52 + 2^31 for the signed high half) by its bit pattern and the bias
+// subtracted exactly; hi * 2^32 + lo then rounds once (a correctly rounded conversion).
+__device__ __forceinline__ double i64_to_f64(int64_t w) {
+    const int lo = static_cast<int>(static_cast<uint32_t>(w));
+    const int hi = static_cast<int>(static_cast<uint32_t>(static_cast<uint64_t>(w) >> 32) ^ 0x80000000u);
+    const double dl = __hiloint2double(0x43300000, lo) - 4503599627370496.0;  // 2^52
+    const double dh = __hiloint2double(0x43300000, hi) - 4503601774854144.0;  // 2^52 + 2^31
+    return fma(dh, 4294967296.0, dl);
+}
+#endif
 
 size_t operand_plane_bytes(OpFmt f, int P, int64_t ld);
 void bind_operand_planes(OperandPlanes& op, OpFmt f, int P, int64_t ld, void* base);
@@ -381,12 +414,14 @@ struct UmmaPlan;
 // images / outputs.
 struct GroupSpec {
     const BlockLayout* L = nullptr;
+    OpFmt fmt = OpFmt::BF16;  // FX and FXS mix in one batch; other formats do not
     GroupInfo info{};
 };
 // Contracts every request of a batch in one persistent launch over all their (block, tile
-// pair) items, requests in ascending order of work. stamps (optional) receives each
+// pair) items (FXS requests in one of their own before it), requests in ascending order of
+// work. stamps (optional) receives each
 // request's completion time (%globaltimer, ns). Synchronises s; timeouts raise.
-void launch_f2_umma_grouped(Ctx& c, OpFmt fmt, double scale_inv, int chunk_stages, const std::vector<GroupSpec>& groups,
+void launch_f2_umma_grouped(Ctx& c, double scale_inv, int chunk_stages, const std::vector<GroupSpec>& groups,
                             cudaStream_t s, std::vector<unsigned long long>* stamps);
 // %globaltimer of the device when the stream reaches this point, written to *dst.
 void launch_timestamp(Ctx& c, unsigned long long* dst, cudaStream_t s);
@@ -437,6 +472,28 @@ size_t fx_vpc_bytes(int n_items);
 // first launch, outside stream capture.
 void fx_prepare();
 void launch_fx(Ctx& c, const FxLaunch& L, cudaStream_t s);
+
+// The same contraction for FXS images (f2_fxs.cu), f2 and counts in one kernel: one item per
+// block, work[0..n_work) in launch order. counter: one int.
+struct FxsLaunch {
+    const uint8_t* images = nullptr;
+    const BlockInfo* work = nullptr;
+    int n_work = 0;
+    int P = 0;
+    double* f2 = nullptr;
+    double* vpair = nullptr;
+    const double* rcp = nullptr;
+    int rcp_max = 0;
+    int* err = nullptr;
+    int* counter = nullptr;
+    int b_base = 0;
+    const GroupInfo* groups = nullptr;
+    int* grp_done = nullptr;
+    unsigned long long* grp_ns = nullptr;
+    const int* grp_items = nullptr;
+};
+void fxs_prepare();
+void launch_fxs(Ctx& c, const FxsLaunch& L, cudaStream_t s);
 
 // chunk_stages: 32-SNP stages per FP32 TMEM chunk (1 or 2).
 UmmaPlan* umma_plan_create(Ctx& c, const OperandPlanes& op, const BlockLayout& L, int chunk_stages);

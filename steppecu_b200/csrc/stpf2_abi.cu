@@ -133,6 +133,20 @@ std::vector<int32_t> make_vpair_units(const std::vector<WorkItem>& items) {
     return u;
 }
 
+namespace {
+// The 32-column tiles of a layout's padded column space (a tile never spans two blocks).
+std::vector<TileInfo> column_tiles(const BlockLayout& L) {
+    std::vector<TileInfo> tiles(static_cast<size_t>(L.ld / kTileK), TileInfo{0, 0});
+    for (int b = 0; b < L.n_block; ++b) {
+        const BlockInfo& bi = L.blocks[b];
+        for (int64_t off = 0; off < bi.k; off += kTileK)
+            tiles[static_cast<size_t>((bi.col + off) / kTileK)] =
+                TileInfo{static_cast<int32_t>(L.snp_begin[b] + off), static_cast<int32_t>(std::min<int64_t>(kTileK, bi.k - off))};
+    }
+    return tiles;
+}
+}  // namespace
+
 size_t operand_plane_bytes(OpFmt f, int P, int64_t ld) {
     if (f == OpFmt::F32) {
         const size_t pl = static_cast<size_t>(P) * static_cast<size_t>(ld);
@@ -341,15 +355,10 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     // 32-column tiles of the padded column space (blocks start on 64-column boundaries,
     // so a tile never spans two blocks).
     p->n_tiles = p->L.ld / 32;
-    std::vector<TileInfo> tiles(static_cast<size_t>(p->n_tiles), TileInfo{0, 0});
+    const std::vector<TileInfo> tiles = column_tiles(p->L);
     std::vector<int32_t> col_snp(static_cast<size_t>(p->L.ld), -1);
     for (int b = 0; b < p->L.n_block; ++b) {
         const BlockInfo& bi = p->L.blocks[b];
-        for (int64_t off = 0; off < (bi.k + 31) / 32 * 32; off += 32) {
-            TileInfo& ti = tiles[static_cast<size_t>((bi.col + off) / 32)];
-            ti.snp0 = static_cast<int32_t>(p->L.snp_begin[b] + off);
-            ti.nvalid = static_cast<int32_t>(std::min<int64_t>(32, bi.k - off));
-        }
         for (int64_t k = 0; k < bi.k; ++k) col_snp[static_cast<size_t>(bi.col + k)] = static_cast<int32_t>(p->L.snp_begin[b] + k);
     }
     upload(p->tiles, tiles, s);
@@ -1767,10 +1776,10 @@ void f2_from_qvn(Ctx& c, const double* Q, const double* V, const double* N, int 
     }
     need(Q && V && N && block_id, "null input");
     DrainOnError drain{c};
-    const BlockLayout L = make_block_layout(block_id, M, n_block);
+    const BlockLayout L = make_block_layout(block_id, M, n_block, !is_fx(fmt_of(precision)));
     const OpFmt fmt = operand_fmt(precision, P, L);
     if (block_sizes) copy_block_sizes(L, block_sizes);
-    DevBuf d_qvn, d_col, d_planes, d_blocks, d_items, d_f2, d_vp;
+    DevBuf d_qvn, d_col, d_tiles, d_planes, d_blocks, d_items, d_f2, d_vp;
     const size_t pm = static_cast<size_t>(P) * M;
     const double *dq = Q, *dv = V, *dn = N;
     if (!qvn_on_device) {
@@ -1783,14 +1792,21 @@ void f2_from_qvn(Ctx& c, const double* Q, const double* V, const double* N, int 
         dv = h + pm;
         dn = h + 2 * pm;
     }
-    upload(d_col, L.snp_col, s);
-    upload(d_blocks, L.blocks, s);
     const size_t ob = operand_plane_bytes(fmt, P, L.ld);
     d_planes.reserve(ob);
-    STPF2_CUDA(cudaMemsetAsync(d_planes.ptr, 0, ob, s));
     OperandPlanes op;
     bind_operand_planes(op, fmt, P, L.ld, d_planes.ptr);
-    launch_feed_qvn(c, dq, dv, dn, P, M, d_col.as<int32_t>(), op, s);
+    std::vector<TileInfo> tiles;
+    if (is_fx(fmt)) {
+        tiles = column_tiles(L);
+        upload(d_tiles, tiles, s);
+        launch_feed_qvn_fx(c, dq, dv, dn, P, d_tiles.as<TileInfo>(), static_cast<int64_t>(tiles.size()), op, s);
+    } else {
+        upload(d_col, L.snp_col, s);
+        upload(d_blocks, L.blocks, s);
+        STPF2_CUDA(cudaMemsetAsync(d_planes.ptr, 0, ob, s));
+        launch_feed_qvn(c, dq, dv, dn, P, M, d_col.as<int32_t>(), op, s);
+    }
     if (precision == STP_PREC_FP32_SIMT) {
         double* f2 = t.f2;
         double* vp = t.vpair;

@@ -405,6 +405,10 @@ void launch_detect_ploidy_canonical(Ctx& c, const uint8_t* packed, uint64_t bpr,
 void launch_feed_qvn(Ctx& c, const double* Q, const double* V, const double* N, int P,
                      int64_t M, const int32_t* snp_col, const OperandPlanes& op, cudaStream_t s);
 
+// The same into fixed-point images (FX, FXS), every one of the layout's n_tiles column tiles.
+void launch_feed_qvn_fx(Ctx& c, const double* Q, const double* V, const double* N, int P, const TileInfo* tiles,
+                        int64_t n_tiles, const OperandPlanes& op, cudaStream_t s);
+
 void launch_f2_simt(Ctx& c, const WorkItem* items, int n_items, const BlockInfo* blocks,
                     const OperandPlanes& op, double* f2, double* vpair, cudaStream_t s);
 

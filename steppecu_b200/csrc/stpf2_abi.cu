@@ -133,20 +133,6 @@ std::vector<int32_t> make_vpair_units(const std::vector<WorkItem>& items) {
     return u;
 }
 
-namespace {
-// The 32-column tiles of a layout's padded column space (a tile never spans two blocks).
-std::vector<TileInfo> column_tiles(const BlockLayout& L) {
-    std::vector<TileInfo> tiles(static_cast<size_t>(L.ld / kTileK), TileInfo{0, 0});
-    for (int b = 0; b < L.n_block; ++b) {
-        const BlockInfo& bi = L.blocks[b];
-        for (int64_t off = 0; off < bi.k; off += kTileK)
-            tiles[static_cast<size_t>((bi.col + off) / kTileK)] =
-                TileInfo{static_cast<int32_t>(L.snp_begin[b] + off), static_cast<int32_t>(std::min<int64_t>(kTileK, bi.k - off))};
-    }
-    return tiles;
-}
-}  // namespace
-
 size_t operand_plane_bytes(OpFmt f, int P, int64_t ld) {
     if (f == OpFmt::F32) {
         const size_t pl = static_cast<size_t>(P) * static_cast<size_t>(ld);
@@ -190,7 +176,7 @@ struct Plan {
     int precision = 0;
     bool detect = false;
     BlockLayout L;
-    DevBuf sel, pop_off, pos, tiles, col_snp, rec_n, rec_nm1, canon, center, blocks, items, own_planes;
+    DevBuf sel, pop_off, pos, tiles, col_snp, rec_n, rec_nm1, canon, center, blocks, items, own_planes, snp_begin;
     DevBuf fold_order;  // per 64-population group, local indices largest first (null: all equal)
     DevBuf fx_table;    // FX: the term table of every (n, a2) (OperandPlanes::fx_table)
     DevBuf row_map;     // kept SNP -> record row (empty: SNP s is record s)
@@ -351,18 +337,17 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     upload(p->rec_n, rn, s);
     upload(p->rec_nm1, rnm1, s);
 
-    p->L = make_block_layout(r.block_id, p->n_snp, r.n_block);
+    p->L = make_block_layout(r.block_id, p->n_snp, r.n_block, false);
     // 32-column tiles of the padded column space (blocks start on 64-column boundaries,
     // so a tile never spans two blocks).
     p->n_tiles = p->L.ld / 32;
-    const std::vector<TileInfo> tiles = column_tiles(p->L);
-    std::vector<int32_t> col_snp(static_cast<size_t>(p->L.ld), -1);
-    for (int b = 0; b < p->L.n_block; ++b) {
-        const BlockInfo& bi = p->L.blocks[b];
-        for (int64_t k = 0; k < bi.k; ++k) col_snp[static_cast<size_t>(bi.col + k)] = static_cast<int32_t>(p->L.snp_begin[b] + k);
-    }
-    upload(p->tiles, tiles, s);
-    upload(p->col_snp, col_snp, s);
+    // The column -> SNP map and the tiles are built on the device from the blocks.
+    upload(p->blocks, p->L.blocks, s);
+    upload(p->snp_begin, p->L.snp_begin, s);
+    p->tiles.reserve(static_cast<size_t>(p->n_tiles) * sizeof(TileInfo));
+    p->col_snp.reserve(static_cast<size_t>(p->L.ld) * sizeof(int32_t));
+    launch_layout_tables(c, p->blocks.as<BlockInfo>(), p->snp_begin.as<int64_t>(), p->L.n_block, p->L.ld,
+                         p->col_snp.as<int32_t>(), p->tiles.as<TileInfo>(), s);
     p->n_sel_pad = (n_sel + 3) / 4 * 4;
     {
         const size_t canon_bytes = std::max<size_t>(static_cast<size_t>((p->n_tiles + 3) / 4) * p->n_sel_pad * 32, 64);
@@ -379,7 +364,6 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     p->bpr = r.geno.bytes_per_record;
     p->words = pitch % 4 == 0 && pitch >= static_cast<uint64_t>((r.geno.n_ind + 3) / 4) &&
                !(r.geno.on_device && reinterpret_cast<uintptr_t>(r.geno.records) % 4 != 0);
-    upload(p->blocks, p->L.blocks, s);
     if (counts_only) return p;  // decode to counts only: no operand planes, no contraction
 
     // A plan cached on the context borrows the shared planes workspace, so building another
@@ -1360,6 +1344,7 @@ stp_ctx* stp_create(int device, stp_status* status) {
         STPF2_CUDA(cudaStreamCreateWithFlags(&c->h2d, cudaStreamNonBlocking));
         STPF2_CUDA(cudaStreamCreateWithFlags(&c->d2h, cudaStreamNonBlocking));
         for (auto& x : c->side) STPF2_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+        pool_open(device);
         out = c.release();
     });
     if (status) *status = st;
@@ -1375,7 +1360,9 @@ void stp_destroy(stp_ctx* ctx) {
             cudaStreamDestroy(s);
         }
     }
+    const int device = ctx->device;
     delete ctx;
+    pool_close(device);
 }
 
 uint64_t stp_launch_count(const stp_ctx* ctx) { return ctx ? ctx->launches.load() : 0; }
@@ -1779,7 +1766,7 @@ void f2_from_qvn(Ctx& c, const double* Q, const double* V, const double* N, int 
     const BlockLayout L = make_block_layout(block_id, M, n_block, !is_fx(fmt_of(precision)));
     const OpFmt fmt = operand_fmt(precision, P, L);
     if (block_sizes) copy_block_sizes(L, block_sizes);
-    DevBuf d_qvn, d_col, d_tiles, d_planes, d_blocks, d_items, d_f2, d_vp;
+    DevBuf d_qvn, d_col, d_begin, d_tiles, d_planes, d_blocks, d_items, d_f2, d_vp;
     const size_t pm = static_cast<size_t>(P) * M;
     const double *dq = Q, *dv = V, *dn = N;
     if (!qvn_on_device) {
@@ -1796,14 +1783,17 @@ void f2_from_qvn(Ctx& c, const double* Q, const double* V, const double* N, int 
     d_planes.reserve(ob);
     OperandPlanes op;
     bind_operand_planes(op, fmt, P, L.ld, d_planes.ptr);
-    std::vector<TileInfo> tiles;
+    upload(d_blocks, L.blocks, s);
     if (is_fx(fmt)) {
-        tiles = column_tiles(L);
-        upload(d_tiles, tiles, s);
-        launch_feed_qvn_fx(c, dq, dv, dn, P, d_tiles.as<TileInfo>(), static_cast<int64_t>(tiles.size()), op, s);
+        const int64_t n_tiles = L.ld / kTileK;
+        upload(d_begin, L.snp_begin, s);
+        d_col.reserve(static_cast<size_t>(L.ld) * sizeof(int32_t));
+        d_tiles.reserve(static_cast<size_t>(n_tiles) * sizeof(TileInfo));
+        launch_layout_tables(c, d_blocks.as<BlockInfo>(), d_begin.as<int64_t>(), n_block, L.ld, d_col.as<int32_t>(),
+                             d_tiles.as<TileInfo>(), s);
+        launch_feed_qvn_fx(c, dq, dv, dn, P, d_tiles.as<TileInfo>(), n_tiles, op, s);
     } else {
         upload(d_col, L.snp_col, s);
-        upload(d_blocks, L.blocks, s);
         STPF2_CUDA(cudaMemsetAsync(d_planes.ptr, 0, ob, s));
         launch_feed_qvn(c, dq, dv, dn, P, M, d_col.as<int32_t>(), op, s);
     }

@@ -1507,8 +1507,8 @@ stp_status stp_snp_keep_mask(stp_ctx* ctx, const stp_geno_view* geno, const int6
             cnt.reserve(static_cast<size_t>(n_pop) * M * 4);
             launch_decode(*p, d_rec, nullptr, nullptr, s, 0, -1, true, cnt.as<uint32_t>());
             const double total = static_cast<double>(pop_offsets[n_pop]);
-            launch_keep_mask_counts(*ctx, cnt.as<uint32_t>(), M, n_pop, M, cols.ref.as<char>(), cols.alt.as<char>(),
-                                    cols.chrom.as<int32_t>(), *filter, total, d_keep.as<uint8_t>(),
+            launch_keep_mask_counts(*ctx, cnt.as<uint32_t>(), M, n_pop, M, p->rec_n.as<double>(), cols.ref.as<char>(),
+                                    cols.alt.as<char>(), cols.chrom.as<int32_t>(), *filter, total, d_keep.as<uint8_t>(),
                                     summary ? d_sum.as<double>() : nullptr, s);
             STPF2_CUDA(cudaMemcpyAsync(keep, d_keep.ptr, static_cast<size_t>(M), cudaMemcpyDeviceToHost, s));
             if (summary)

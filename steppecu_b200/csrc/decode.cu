@@ -748,10 +748,22 @@ decode_canon_kernel(const uint64_t* __restrict__ canon, int64_t n_tiles, int64_t
             }
         }
         if (cnt_packed) {
+            // A chunk's eight columns are one block's, so its SNPs are consecutive while they
+            // last: a lane's 32 bytes as two 16-byte stores (a sector each) where the row is
+            // aligned for them, instead of eight stores of 4 bytes to 32 sectors each
+            // (the decode of 200 populations x 600,000 SNPs to counts 458 -> 260 us).
+            const int4 ca = __ldg(reinterpret_cast<const int4*>(col_snp + col0));
+            const int4 cb = __ldg(reinterpret_cast<const int4*>(col_snp + col0) + 1);
+            const int32_t sc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+            uint32_t* row = cnt_packed + static_cast<int64_t>(i) * cnt_ld;
+            if (sc[0] >= 0 && sc[7] >= 0 && (reinterpret_cast<uintptr_t>(row + sc[0]) & 15) == 0) {
+                uint4* o = reinterpret_cast<uint4*>(row + sc[0]);
+                o[0] = make_uint4(cnt[0], cnt[kCntCol], cnt[2 * kCntCol], cnt[3 * kCntCol]);
+                o[1] = make_uint4(cnt[4 * kCntCol], cnt[5 * kCntCol], cnt[6 * kCntCol], cnt[7 * kCntCol]);
+            } else {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const int32_t s = __ldg(col_snp + col0 + c);
-                if (s >= 0) cnt_packed[static_cast<int64_t>(i) * cnt_ld + s] = cnt[c * kCntCol];
+                for (int c = 0; c < 8; ++c)
+                    if (sc[c] >= 0) row[sc[c]] = cnt[c * kCntCol];
             }
         }
         if (!op.planes) continue;

@@ -391,7 +391,8 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
 // centres are indexed from t0, for the pipelined host-buffer path; detect runs the ploidy
 // pass first (it reads the first min(1000, M) SNPs).
 void launch_decode(Plan& p, const uint8_t* d_records, int32_t* cnt_ac2, int32_t* cnt_n, cudaStream_t s,
-                   int64_t t0 = 0, int64_t t1 = -1, bool detect = true, uint32_t* cnt_packed = nullptr) {
+                   int64_t t0 = 0, int64_t t1 = -1, bool detect = true, uint32_t* cnt_packed = nullptr,
+                   int64_t cnt_ld = 0) {
     Ctx& c = *p.ctx;
     if (p.n_snp <= 0) return;
     if (t1 < 0) t1 = p.n_tiles;
@@ -424,7 +425,7 @@ void launch_decode(Plan& p, const uint8_t* d_records, int32_t* cnt_ac2, int32_t*
     if (cnt_packed) {
         a.op.planes = nullptr;
         a.cnt_packed = cnt_packed;
-        a.cnt_ld = p.n_snp;
+        a.cnt_ld = cnt_ld;
     }
     a.fold_order = p.fold_order.as<int32_t>();
     launch_decode_canon(c, a, s);
@@ -1503,11 +1504,12 @@ stp_status stp_snp_keep_mask(stp_ctx* ctx, const stp_geno_view* geno, const int6
                 d_rec = rec.as<uint8_t>();
             }
             std::unique_ptr<Plan> p = build_plan(*ctx, r, pitch, nullptr, false, /*counts_only=*/true);
+            const int64_t ld = (M + 3) / 4 * 4;  // rows 16-byte aligned: vector stores
             DevBuf cnt;
-            cnt.reserve(static_cast<size_t>(n_pop) * M * 4);
-            launch_decode(*p, d_rec, nullptr, nullptr, s, 0, -1, true, cnt.as<uint32_t>());
+            cnt.reserve(static_cast<size_t>(n_pop) * ld * 4);
+            launch_decode(*p, d_rec, nullptr, nullptr, s, 0, -1, true, cnt.as<uint32_t>(), ld);
             const double total = static_cast<double>(pop_offsets[n_pop]);
-            launch_keep_mask_counts(*ctx, cnt.as<uint32_t>(), M, n_pop, M, p->rec_n.as<double>(), cols.ref.as<char>(),
+            launch_keep_mask_counts(*ctx, cnt.as<uint32_t>(), ld, n_pop, M, p->rec_n.as<double>(), cols.ref.as<char>(),
                                     cols.alt.as<char>(), cols.chrom.as<int32_t>(), *filter, total, d_keep.as<uint8_t>(),
                                     summary ? d_sum.as<double>() : nullptr, s);
             STPF2_CUDA(cudaMemcpyAsync(keep, d_keep.ptr, static_cast<size_t>(M), cudaMemcpyDeviceToHost, s));

@@ -549,6 +549,7 @@ transpose_pa_kernel(const RecordView v, int64_t n_ind,
                 if (g[m] >= 0) canon[(q * n_sel + g[m]) * 4 + sub] = out[m];
         }
     }
+    pdl_wait();  // the ploidy pass it may overlap: the decode follows both
 }
 
 // Pass 2: one CTA per (64 populations, quad of 4 column tiles), in two phases.
@@ -654,6 +655,7 @@ decode_canon_kernel(const uint64_t* __restrict__ canon, int64_t n_tiles, int64_t
                     OperandPlanes op, int32_t* __restrict__ cnt_ac2, int32_t* __restrict__ cnt_n,
                     const int32_t* __restrict__ umap, const double* __restrict__ center_snp,
                     uint32_t* __restrict__ cnt_packed, int64_t cnt_ld, const int32_t* __restrict__ fold_order) {
+    pdl_trigger();
     extern __shared__ uint32_t s_cnt[];
     __shared__ double s_center[4 * kCenterPitch];
     const int64_t q = blockIdx.x;
@@ -966,6 +968,7 @@ constexpr int kPlWords = 8, kPlThreads = 1024;
 __global__ void __launch_bounds__(kPlThreads)
 detect_ploidy_words_kernel(const RecordView v, int64_t window, int64_t n_ind, const int32_t* __restrict__ pos,
                            uint32_t* __restrict__ sel) {
+    pdl_trigger();  // the transpose needs nothing from here
     __shared__ uint32_t s_het[kPlWords];
     const int k = threadIdx.x % kPlWords;
     const int64_t w = static_cast<int64_t>(blockIdx.x) * kPlWords + k;
@@ -1068,21 +1071,21 @@ namespace {
 template <int kGran>
 void transpose_gran(Ctx& c, unsigned n_quads, const RecordView& v, int64_t n_ind, const TileInfo* tiles, int64_t n_tiles,
                     const int32_t* pos, int64_t n_sel, int64_t n_slices, uint64_t* canon, double* center,
-                    const int32_t* row_map, cudaStream_t s) {
+                    const int32_t* row_map, cudaStream_t s, bool early) {
     static std::atomic<bool> attr_set[64] = {};  // per device ordinal
     if (c.device < 0 || c.device >= 64 || !attr_set[c.device]) {
         STPF2_CUDA(cudaFuncSetAttribute(transpose_pa_kernel<kGran>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(kTransSmemBytes)));
         if (c.device >= 0 && c.device < 64) attr_set[c.device] = true;
     }
-    transpose_pa_kernel<kGran><<<n_quads, kTransThreads, kTransSmemBytes, s>>>(v, n_ind, tiles, n_tiles, pos, n_sel,
-                                                                               n_slices, canon, center, row_map);
+    launch_kernel_on(transpose_pa_kernel<kGran>, n_quads, kTransThreads, kTransSmemBytes, s, early, v, n_ind, tiles, n_tiles,
+                     pos, n_sel, n_slices, canon, center, row_map);
 }
 }  // namespace
 
 void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_t bpr, int64_t n_ind,
                          const TileInfo* tiles, int64_t n_tiles, const int32_t* pos, int64_t n_sel, uint64_t* canon,
-                         double* center, cudaStream_t s, const int32_t* row_map) {
+                         double* center, cudaStream_t s, const int32_t* row_map, bool early) {
     if (n_tiles <= 0) return;
     const RecordView v = record_view(records, pitch, bpr, n_ind);
     // Every row starts where the pitch and the base put it: the form is their common alignment.
@@ -1090,11 +1093,11 @@ void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_
     const unsigned n_quads = static_cast<unsigned>((n_tiles + 3) / 4);
     const int64_t n_slices = std::max<int64_t>(1, (n_ind + kSliceWords * 16 - 1) / (kSliceWords * 16));
     if (align % 16 == 0)
-        transpose_gran<16>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s);
+        transpose_gran<16>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s, early);
     else if (align % 4 == 0)
-        transpose_gran<4>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s);
+        transpose_gran<4>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s, early);
     else
-        transpose_gran<1>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s);
+        transpose_gran<1>(c, n_quads, v, n_ind, tiles, n_tiles, pos, n_sel, n_slices, canon, center, row_map, s, early);
     STPF2_CUDA(cudaGetLastError());
     c.launches++;
 }

@@ -102,7 +102,7 @@ struct FxArgs {
     const double* rcp;  // rcp[k] = 1/k, k = 0..rcp_max (rcp[0] = 0)
     int rcp_max;
     int* err;
-    int* next_item;  // work-item (f2) or unit (vpair) counter, zero at launch
+    int* next_item;  // work-item (f2) or unit (vpair) counter, zero at launch and left zero
     const int32_t* units;  // vpair units: first item of each, as an index past unit_base
     int n_units;
     int unit_base;
@@ -355,6 +355,14 @@ __device__ __forceinline__ void stamp(const FxArgs& a, int grp, int lane) {
     }
 }
 
+// Counts of the vpair kernel, which may end while this one already runs: through L2, in
+// program order after the wait for it.
+__device__ __forceinline__ int32_t ld_cg(const int32_t* p) {
+    int32_t v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ void st_cs_v2(double* p, double x, double y) {
     asm volatile("st.global.cs.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(x), "d"(y) : "memory");
 }
@@ -470,7 +478,7 @@ __device__ void fx_epilogue(const FxArgs& a, FxCtl* ctl, uint32_t tmem, int warp
         for (int q8 = 0; q8 < kCols / 8; ++q8) {
             int32_t vpi[8];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) vpi[c] = __ldg(vpt + (q8 * 8 + c) * kTile + lane);
+            for (int c = 0; c < 8; ++c) vpi[c] = ld_cg(vpt + (q8 * 8 + c) * kTile + lane);
             double f8[8], v8[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
@@ -533,6 +541,9 @@ f2_fx_kernel(const __grid_constant__ FxArgs a) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
+    // Launched programmatically after the vpair kernel, which lets it start once the decode is
+    // complete: the images are ready, only the epilogue waits for the counts.
+    if (warp >= kEpiWarp0) pdl_wait();
     if (warp < kEpiWarp0) {
         if (warp == 0 && lane == 0) fx_producer<kGrouped>(a, smem, ctl);
         if (warp == 1 && lane == 0) fx_issuer<kGrouped>(a, smem, ctl, tmem);
@@ -543,6 +554,7 @@ f2_fx_kernel(const __grid_constant__ FxArgs a) {
     __syncthreads();
     tc_fence_after();
     if (warp == 1) tmem_dealloc(tmem, kTmemCols);
+    if (threadIdx.x == 0) reset_counter(a.next_item);
 }
 
 constexpr size_t kFxSmemBytes = kStages * kStageBytes + kCtlBytes + 1024;
@@ -770,6 +782,8 @@ __global__ void __launch_bounds__(kVpThreads, 1) vpair_fx_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
+    pdl_wait();  // the decode's M tiles
+    pdl_trigger();
     if (warp < 2) {
         if (warp == 0 && lane == 0) vp_producer<kGrouped>(a, smem, ctl);
         if (warp == 1 && lane == 0) vp_issuer<kGrouped>(a, smem, ctl, tmem);
@@ -780,6 +794,7 @@ __global__ void __launch_bounds__(kVpThreads, 1) vpair_fx_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     if (warp == 1) tmem_dealloc(tmem, kTmemCols);
+    if (threadIdx.x == 0) reset_counter(a.next_item);
 }
 
 constexpr size_t kVpSmemBytes = kVpStages * kVpStageBytes + kCtlBytes + 1024;
@@ -833,25 +848,15 @@ void launch_fx(Ctx& c, const FxLaunch& L, cudaStream_t s) {
     if (!L.units || L.n_units <= 0) fail(STP_RUNTIME_ERROR, "fixed-point contraction without vpair units");
     const int grid = std::min(c.sm_count, L.n_items);
     // Two work counters: vpair units, then f2 items.
-    STPF2_CUDA(cudaMemsetAsync(L.counters, 0, 2 * sizeof(int), s));
     a.next_item = L.counters;
     const int vp_grid = std::min(c.sm_count, L.n_units);
-    if (L.groups) vpair_fx_kernel<true><<<vp_grid, kVpThreads, kVpSmemBytes, s>>>(a);
-    else vpair_fx_kernel<false><<<vp_grid, kVpThreads, kVpSmemBytes, s>>>(a);
-    STPF2_CUDA(cudaGetLastError());
+    launch_kernel_on(L.groups ? vpair_fx_kernel<true> : vpair_fx_kernel<false>, static_cast<unsigned>(vp_grid), kVpThreads,
+                     kVpSmemBytes, s, L.early, a);
     c.launches++;
-    a.next_item = L.counters + 1;
+    a.next_item = L.counters + 2;
     a.withhold = c.fx_tuning.withhold_stage;  // test hook: starves the f2 kernel's issuer
-    if (L.groups) f2_fx_kernel<true><<<grid, kThreads, kFxSmemBytes, s>>>(a);
-    else f2_fx_kernel<false><<<grid, kThreads, kFxSmemBytes, s>>>(a);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        cudaFuncAttributes fa{};
-        cudaFuncGetAttributes(&fa, f2_fx_kernel<false>);
-        fail(STP_CUDA_ERROR, std::string("f2_fx_kernel launch: ") + cudaGetErrorString(e) + " (regs " +
-                                 std::to_string(fa.numRegs) + ", dyn smem " + std::to_string(kFxSmemBytes) + ", local " +
-                                 std::to_string(fa.localSizeBytes) + ")");
-    }
+    launch_kernel_on(L.groups ? f2_fx_kernel<true> : f2_fx_kernel<false>, static_cast<unsigned>(grid), kThreads,
+                     kFxSmemBytes, s, true, a);
     c.launches++;
 }
 

@@ -63,7 +63,7 @@ struct FxsArgs {
     const double* rcp;  // rcp[k] = 1/k
     int rcp_max;
     int* err;
-    int* next;  // work counter, zero at launch
+    int* next;  // work counter, zero at launch and left zero
     int b_base;
     unsigned long long timeout_ns;
     long long withhold;  // test hook: the producer stops before its stage of this index
@@ -363,6 +363,7 @@ __global__ void __launch_bounds__(kThreads, 1) f2_fxs_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
+    pdl_wait();  // the decode's images
     if (warp < 2) {
         if (warp == 0 && lane == 0) fxs_producer<kGrouped>(a, smem, ctl);
         if (warp == 1 && lane == 0) fxs_issuer<kGrouped>(a, smem, ctl, tmem);
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) f2_fxs_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     if (warp == 1) tmem_dealloc(tmem, kTmemCols);
+    if (threadIdx.x == 0) reset_counter(a.next);
 }
 
 }  // namespace
@@ -404,10 +406,8 @@ void launch_fxs(Ctx& c, const FxsLaunch& L, cudaStream_t s) {
     a.grp_ns = L.grp_ns;
     a.grp_items = L.grp_items;
     const int grid = std::min(c.sm_count, L.n_work);
-    STPF2_CUDA(cudaMemsetAsync(L.counter, 0, sizeof(int), s));
-    if (L.groups) f2_fxs_kernel<true><<<grid, kThreads, kFxsSmemBytes, s>>>(a);
-    else f2_fxs_kernel<false><<<grid, kThreads, kFxsSmemBytes, s>>>(a);
-    STPF2_CUDA(cudaGetLastError());
+    launch_kernel_on(L.groups ? f2_fxs_kernel<true> : f2_fxs_kernel<false>, static_cast<unsigned>(grid), kThreads,
+                     kFxsSmemBytes, s, L.early, a);
     c.launches++;
 }
 

@@ -571,6 +571,7 @@ void upload_control(Ctx& c, UmmaPlan& p, const BlockLayout& L) {
     p.err.reserve(16);
     p.counter.reserve(16);
     STPF2_CUDA(cudaMemsetAsync(p.err.ptr, 0, 16, c.stream));
+    STPF2_CUDA(cudaMemsetAsync(p.counter.ptr, 0, 16, c.stream));
     const std::vector<double> rcp = reciprocals(p.rcp_max = longest_block(L));
     p.rcp.reserve(rcp.size() * sizeof(double));
     STPF2_CUDA(cudaMemcpyAsync(p.rcp.ptr, rcp.data(), rcp.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
@@ -653,11 +654,11 @@ UmmaPlan* umma_plan_create(Ctx& c, const OperandPlanes& op, const BlockLayout& L
 void umma_plan_destroy(UmmaPlan* p) { delete p; }
 
 void launch_umma_items(Ctx& c, UmmaPlan* p, const WorkItem* items, int n_items, double* f2, double* vpair,
-                       cudaStream_t s, int b_base = 0, int b0 = -1, int b1 = -1);
+                       cudaStream_t s, int b_base = 0, int b0 = -1, int b1 = -1, bool early = false);
 
 // n items of an FXS work list.
 void launch_fxs_items(Ctx& c, UmmaPlan* p, const BlockInfo* work, int n, double* f2, double* vpair, cudaStream_t s,
-                      int b_base) {
+                      int b_base, bool early = false) {
     FxsLaunch L;
     L.images = p->images;
     L.work = work;
@@ -670,12 +671,13 @@ void launch_fxs_items(Ctx& c, UmmaPlan* p, const BlockInfo* work, int n, double*
     L.err = p->err.as<int>();
     L.counter = p->counter.as<int>();
     L.b_base = b_base;
+    L.early = early;
     launch_fxs(c, L, s);
 }
 
-void launch_f2_umma(Ctx& c, UmmaPlan* p, double* f2, double* vpair, cudaStream_t s, bool per_block) {
+void launch_f2_umma(Ctx& c, UmmaPlan* p, double* f2, double* vpair, cudaStream_t s, bool per_block, bool early) {
     if (!p || p->n_items <= 0) return;
-    if (p->fmt == OpFmt::FXS) return launch_fxs_items(c, p, p->work.as<BlockInfo>(), p->n_items, f2, vpair, s, 0);
+    if (p->fmt == OpFmt::FXS) return launch_fxs_items(c, p, p->work.as<BlockInfo>(), p->n_items, f2, vpair, s, 0, early);
     if (per_block) {  // comparison form: one launch per jackknife block
         for (size_t b = 0; b + 1 < p->block_item_off.size(); ++b) {
             const int n = p->block_item_off[b + 1] - p->block_item_off[b];
@@ -685,7 +687,7 @@ void launch_f2_umma(Ctx& c, UmmaPlan* p, double* f2, double* vpair, cudaStream_t
         }
         return;
     }
-    launch_umma_items(c, p, p->items.as<WorkItem>(), p->n_items, f2, vpair, s);
+    launch_umma_items(c, p, p->items.as<WorkItem>(), p->n_items, f2, vpair, s, 0, -1, -1, early);
 }
 
 void launch_f2_umma_blocks(Ctx& c, UmmaPlan* p, int b0, int b1, double* f2, double* vpair, cudaStream_t s,
@@ -702,7 +704,7 @@ void launch_f2_umma_blocks(Ctx& c, UmmaPlan* p, int b0, int b1, double* f2, doub
 // b0 < 0: items is the whole costliest-first list; otherwise the block_items of blocks
 // b0..b1-1.
 void launch_umma_items(Ctx& c, UmmaPlan* p, const WorkItem* items, int n_items, double* f2, double* vpair,
-                       cudaStream_t s, int b_base, int b0, int b1) {
+                       cudaStream_t s, int b_base, int b0, int b1, bool early) {
     if (p->fmt == OpFmt::FX) {
         FxLaunch L;
         L.images = p->images;
@@ -729,6 +731,7 @@ void launch_umma_items(Ctx& c, UmmaPlan* p, const WorkItem* items, int n_items, 
         L.err = p->err.as<int>();
         L.counters = p->counter.as<int>();
         L.b_base = b_base;
+        L.early = early;
         launch_fx(c, L, s);
         return;
     }

@@ -8,8 +8,8 @@
 // taken once per device with cudaGetSymbolAddress. The reference has no counterpart: its
 // backends allocate per call.
 //
-// What must start at a fixed value is set by the call itself with cudaMemsetAsync: the
-// file-row map (-1 = not selected) and the error flag (0). Everything else in the scratch
+// What must start at a fixed value is set by the call's first kernel: the file-row map (-1 =
+// not selected) and the error flag (0). Everything else in the scratch
 // is written before it is read within the same call. The scratch is shared by every call
 // on a device, so calls whose work overlaps in time (other host threads, other streams)
 // race on it and must be serialised by the caller.
@@ -47,11 +47,15 @@ __global__ void noalloc_select_kernel(const int64_t* __restrict__ sel_rows, int6
     if (atomicCAS(pos + row, -1, static_cast<int32_t>(g)) != -1) atomicExch(err, 1);
 }
 
-// Contiguous column space (no block padding): tile t holds SNPs 32t .. 32t+31.
+// Contiguous column space (no block padding): tile t holds SNPs 32t .. 32t+31. Also the start
+// of the row map (no row selected) and of the error flag.
 __global__ void noalloc_layout_kernel(int64_t n_snp, int64_t n_tiles, TileInfo* __restrict__ tiles,
                                       int32_t* __restrict__ col_snp, const int64_t* __restrict__ po64,
-                                      int32_t* __restrict__ po32, int P) {
+                                      int32_t* __restrict__ po32, int P, int32_t* __restrict__ pos, int64_t n_pos,
+                                      int* err) {
     const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k < n_pos) pos[k] = -1;
+    if (k == 0) *err = 0;
     if (k < n_tiles * kTileK) col_snp[k] = k < n_snp ? static_cast<int32_t>(k) : -1;
     if (k < n_tiles) {
         const int64_t rem = n_snp - k * kTileK;
@@ -140,21 +144,20 @@ void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, uin
     STPF2_CUDA(cudaMemcpyAsync(d_po64, pop_offsets, static_cast<size_t>(P + 1) * 8, cudaMemcpyHostToDevice, s));
     if (d_pl)
         STPF2_CUDA(cudaMemcpyAsync(d_pl, sample_ploidy, static_cast<size_t>(n_sel) * 4, cudaMemcpyHostToDevice, s));
-    STPF2_CUDA(cudaMemsetAsync(d_pos, 0xFF, static_cast<size_t>(n_ind16) * 4, s));  // -1: not selected
-    STPF2_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), s));
+    const int64_t layout_n = std::max<int64_t>({n_tiles * kTileK, P + 1, n_ind16});
+    noalloc_layout_kernel<<<static_cast<unsigned>((layout_n + 255) / 256), 256, 0, s>>>(
+        n_snp, n_tiles, d_tiles, d_col_snp, d_po64, d_po32, P, d_pos, n_ind16, d_err);
+    STPF2_CUDA(cudaGetLastError());
+    c.launches++;
     if (n_sel > 0) {
         noalloc_select_kernel<<<static_cast<unsigned>((n_sel + 255) / 256), 256, 0, s>>>(
             d_sel_rows, n_sel, d_pl, mode_ploidy, d_desc, d_pos, d_err);
         STPF2_CUDA(cudaGetLastError());
         c.launches++;
     }
-    const int64_t layout_n = std::max<int64_t>(n_tiles * kTileK, P + 1);
-    noalloc_layout_kernel<<<static_cast<unsigned>((layout_n + 255) / 256), 256, 0, s>>>(
-        n_snp, n_tiles, d_tiles, d_col_snp, d_po64, d_po32, P);
-    STPF2_CUDA(cudaGetLastError());
-    c.launches++;
     if (detect) launch_detect_ploidy_words(c, d_records, pitch, bpr, n_snp, n_ind, d_pos, d_desc, s);
-    launch_transpose_pa(c, d_records, pitch, bpr, n_ind, d_tiles, n_tiles, d_pos, n_sel_pad, d_canon, nullptr, s);
+    launch_transpose_pa(c, d_records, pitch, bpr, n_ind, d_tiles, n_tiles, d_pos, n_sel_pad, d_canon, nullptr, s, nullptr,
+                        detect);
     CanonDecodeArgs a;
     a.canon = d_canon;
     a.n_tiles = n_tiles;

@@ -404,8 +404,9 @@ void launch_decode(Plan& p, const uint8_t* d_records, int32_t* cnt_ac2, int32_t*
     if (t1 <= t0) return;
     const bool counts = cnt_ac2 || cnt_packed;
     double* center = is_fx(p.op.fmt) || counts ? nullptr : p.center_ptr + t0 * kTileK;
+    const bool early = p.detect && detect;  // the transpose overlaps the ploidy pass
     launch_transpose_pa(c, rec, p.pitch, p.bpr, p.n_ind, p.tiles.as<TileInfo>() + t0, t1 - t0, p.pos.as<int32_t>(),
-                        p.n_sel_pad, p.canon_ptr, center, s, p.row_map.as<int32_t>());
+                        p.n_sel_pad, p.canon_ptr, center, s, p.row_map.as<int32_t>(), early);
     CanonDecodeArgs a;
     a.canon = p.canon_ptr;
     a.n_tiles = t1 - t0;
@@ -455,7 +456,7 @@ void run_plan(Plan& p, const uint8_t* d_records, double* d_f2, double* d_vpair, 
     if (p.precision == STP_PREC_FP32_SIMT)
         launch_f2_simt(c, p.items.as<WorkItem>(), p.n_items, p.blocks.as<BlockInfo>(), p.op, d_f2, d_vpair, s);
     else
-        launch_f2_umma(c, p.umma, d_f2, d_vpair, s, p.per_block);
+        launch_f2_umma(c, p.umma, d_f2, d_vpair, s, p.per_block, !tev);
     if (tev) STPF2_CUDA(cudaEventRecord((*tev)[2], s));
 }
 

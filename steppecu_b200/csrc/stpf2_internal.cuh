@@ -321,6 +321,39 @@ inline OpFmt operand_fmt(int precision, int P, const BlockLayout& L) {
 }
 
 #ifdef __CUDACC__
+// Programmatic dependent launch: a kernel launched with `early` may start once every CTA of the
+// kernel before it on the stream has called pdl_trigger (or ended), and pdl_wait holds it until
+// that kernel has completed. What runs before pdl_wait must touch nothing that the kernel
+// before it writes. On a kernel launched plainly both do nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... K, class... A>
+void launch_kernel_on(void (*kernel)(K...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, bool early,
+                      A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    STPF2_CUDA(cudaLaunchKernelEx(&cfg, kernel, K(args)...));
+}
+
+// Leaves a persistent kernel's work counter at zero for its next launch: the last CTA to get
+// here resets it (counter[0]: the work, counter[1]: the CTAs that have ended).
+__device__ __forceinline__ void reset_counter(int* counter) {
+    __threadfence();
+    if (atomicAdd(counter + 1, 1) == static_cast<int>(gridDim.x) - 1) {
+        counter[0] = 0;
+        counter[1] = 0;
+    }
+}
+
 // int64 -> FP64 without a conversion instruction: each 32-bit half is placed in the
 // mantissa of 2^52 (2^52 + 2^31 for the signed high half) by its bit pattern and the bias
 // subtracted exactly; hi * 2^32 + lo then rounds once (a correctly rounded conversion).
@@ -394,7 +427,7 @@ void launch_detect_ploidy_pa(Ctx& c, const uint8_t* records, uint64_t pitch, int
 // tiles name (a kept-SNP compaction).
 void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_t bpr, int64_t n_ind,
                          const TileInfo* tiles, int64_t n_tiles, const int32_t* pos, int64_t n_sel, uint64_t* canon,
-                         double* center, cudaStream_t s, const int32_t* row_map = nullptr);
+                         double* center, cudaStream_t s, const int32_t* row_map = nullptr, bool early = false);
 // Canonical individual-major tile -> SNP-major records (pitch >= ceil(n_ind / 4)).
 void launch_canonical_to_records(Ctx& c, const uint8_t* packed, uint64_t bpr, int64_t n_snp, int64_t n_ind,
                                  uint8_t* records, uint64_t pitch, cudaStream_t s);
@@ -461,7 +494,7 @@ void launch_copy_union_ploidy(Ctx& c, uint32_t* desc, const int32_t* umap, int64
                               cudaStream_t s);
 
 // The fixed-point contraction (f2_fx.cu): vpair_fx_kernel then f2_fx_kernel over the same
-// items. vpc holds fx_vpc_bytes(n_items); counters two ints; groups non-null for a batch.
+// items. vpc holds fx_vpc_bytes(n_items); groups non-null for a batch.
 struct FxLaunch {
     const uint8_t* images = nullptr;
     const uint8_t* mplanes = nullptr;
@@ -479,8 +512,9 @@ struct FxLaunch {
     const double* rcp = nullptr;
     int rcp_max = 0;
     int* err = nullptr;
-    int* counters = nullptr;
+    int* counters = nullptr;  // two pairs (work, ended CTAs), vpair's and f2's; zero, and left zero
     int b_base = 0;
+    bool early = false;  // the kernel before on the stream is the decode (programmatic launch)
     const GroupInfo* groups = nullptr;
     int* grp_done = nullptr;
     unsigned long long* grp_ns = nullptr;
@@ -493,7 +527,7 @@ void fx_prepare();
 void launch_fx(Ctx& c, const FxLaunch& L, cudaStream_t s);
 
 // The same contraction for FXS images (f2_fxs.cu), f2 and counts in one kernel: one item per
-// block, work[0..n_work) in launch order. counter: one int.
+// block, work[0..n_work) in launch order.
 struct FxsLaunch {
     const uint8_t* images = nullptr;
     const BlockInfo* work = nullptr;
@@ -504,8 +538,9 @@ struct FxsLaunch {
     const double* rcp = nullptr;
     int rcp_max = 0;
     int* err = nullptr;
-    int* counter = nullptr;
+    int* counter = nullptr;  // a pair (work, ended CTAs); zero, and left zero
     int b_base = 0;
+    bool early = false;  // the kernel before on the stream is the decode (programmatic launch)
     const GroupInfo* groups = nullptr;
     int* grp_done = nullptr;
     unsigned long long* grp_ns = nullptr;
@@ -521,7 +556,9 @@ inline int chunk_stages_of(int precision) { return precision == STP_PREC_SPLIT_F
 void umma_plan_destroy(UmmaPlan* p);
 // per_block: one launch per jackknife block instead of one persistent launch over all
 // blocks (the comparison form of the grouped schedule).
-void launch_f2_umma(Ctx& c, UmmaPlan* p, double* f2, double* vpair, cudaStream_t s, bool per_block = false);
+// early: the kernel before on the stream is the plan's decode.
+void launch_f2_umma(Ctx& c, UmmaPlan* p, double* f2, double* vpair, cudaStream_t s, bool per_block = false,
+                    bool early = false);
 // The tile pairs of blocks [b0, b1) only, in one launch.
 // Blocks [b0, b1) only; rebase: f2 / vpair point at block b0's slab (a buffer of b1 - b0
 // slabs) instead of the whole tensor.

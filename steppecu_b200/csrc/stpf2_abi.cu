@@ -1215,18 +1215,22 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
         a.cnt_ld = cnt_ld;
         launch_decode_canon(c, a, s);
     }
-    for (size_t m = 0; m < mem.size(); ++m)
-        launch_layout_tables(c, reinterpret_cast<const BlockInfo*>(T + mo[m].blocks),
-                             reinterpret_cast<const int64_t*>(T + mo[m].begin), mem[m].L.n_block, mem[m].L.ld,
-                             reinterpret_cast<int32_t*>(T + mo[m].cols), reinterpret_cast<TileInfo*>(T + mo[m].tiles), s);
-
-    // Waves of requests whose operand images (and device-side outputs) fit together.
-    STPF2_CUDA(cudaStreamSynchronize(s));
-    size_t free_b = 0, total_b = 0;
-    STPF2_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const size_t held = c.ws_batch.bytes + c.ws_f2.bytes + c.ws_vpair.bytes + c.ws_vpc.bytes;  // reusable here
-    const size_t avail = free_b + held;
-    const size_t budget = avail > (size_t(2) << 30) ? (avail - (size_t(2) << 30)) * 9 / 10 : 0;
+    // Waves of requests whose operand images (and device-side outputs) fit together. One wave
+    // that fits in what earlier calls left needs no look at the free memory.
+    size_t need_img = 0, need_out = 0, need_vpc = 0;
+    for (const BatchMember& m : mem) {
+        need_img += m.img_bytes;
+        need_out += m.out_bytes / 2;
+        need_vpc += m.vpc_bytes;
+    }
+    size_t budget = SIZE_MAX;
+    if (need_img > c.ws_batch.bytes || need_out > std::min(c.ws_f2.bytes, c.ws_vpair.bytes) || need_vpc > c.ws_vpc.bytes) {
+        size_t free_b = 0, total_b = 0;
+        STPF2_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        const size_t held = c.ws_batch.bytes + c.ws_f2.bytes + c.ws_vpair.bytes + c.ws_vpc.bytes;  // reusable here
+        const size_t avail = free_b + held;
+        budget = avail > (size_t(2) << 30) ? (avail - (size_t(2) << 30)) * 9 / 10 : 0;
+    }
     std::vector<std::vector<size_t>> waves(1);
     size_t acc = 0;
     for (size_t m = 0; m < mem.size(); ++m) {
@@ -1265,9 +1269,14 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
             p.op.fx_table = d_fxtab;
             p.op.fx_table_ld = static_cast<int32_t>(2 * n_max + 1);
             io += p.img_bytes;
+            // The request's column map, on its emission's stream: 25 such launches one after
+            // another on the main stream took 196 us of a 24-request batch.
+            const cudaStream_t es = fork.next();
+            launch_layout_tables(c, reinterpret_cast<const BlockInfo*>(T + q.blocks), reinterpret_cast<const int64_t*>(T + q.begin),
+                                 p.L.n_block, p.L.ld, reinterpret_cast<int32_t*>(T + q.cols),
+                                 reinterpret_cast<TileInfo*>(T + q.tiles), es);
             launch_emit_counts(c, d_counts, cnt_ld, M, reinterpret_cast<const int32_t*>(T + q.upop), p.P, p.L.ld / kTileK,
-                               reinterpret_cast<const int32_t*>(T + q.cols), d_center_u, d_rn, d_rnm1, p.op,
-                               fork.next());
+                               reinterpret_cast<const int32_t*>(T + q.cols), d_center_u, d_rn, d_rnm1, p.op, es);
             double* f2 = o.f2;
             double* vp = o.vpair;
             if (!o.on_device) {

@@ -133,6 +133,10 @@ __device__ __forceinline__ bool waitb(unsigned long long* b, uint32_t parity, Fx
     return wait_bounded(b, parity, &ctl->abort, a.err, a.timeout_ns, honour_abort);
 }
 
+__device__ __forceinline__ bool waitw(unsigned long long* b, uint32_t parity, FxCtl* ctl, const FxArgs& a, int lane) {
+    return wait_warp(b, parity, &ctl->abort, a.err, a.timeout_ns, lane);
+}
+
 __device__ __forceinline__ int stages_of(int k, int per) { return (k + per - 1) / per; }
 
 // The MMA width of a tile pair: the column tile's populations rounded up to the N step of
@@ -203,81 +207,96 @@ __device__ __forceinline__ void copy_side(uint8_t* dst, const uint8_t* img, cons
     bulk_load(dst + kImg, mt, b, bar);
 }
 
+// The whole of warp 0.
 template <bool kGrouped>
-__device__ void fx_producer(const FxArgs& a, uint8_t* smem, FxCtl* ctl) {
+__device__ void fx_producer(const FxArgs& a, uint8_t* smem, FxCtl* ctl, int lane) {
     uint32_t g = 0;
-    for (uint32_t gi = 0;; ++gi) {
+    bool stopped = false;
+    for (uint32_t gi = 0; !stopped; ++gi) {
         bool ok = true;
-        const int it = take_item(a, ctl, gi, ok);
-        if (!ok) goto abort;
-        if (it < 0) break;
-        {
-            const WorkItem w = a.items[it];
-            const BlockInfo bi = a.blocks[w.blk];
-            const int nst = stages_of(bi.k, kStageK);
-            const bool diag = w.ti == w.tj;
-            const uint8_t* images = a.images;
-            const uint8_t* mplanes = a.mplanes;
-            int64_t n_ck = a.n_ck;
-            if constexpr (kGrouped) {
-                images = a.groups[bi.grp].images;
-                mplanes = a.groups[bi.grp].mplanes;
-                n_ck = a.groups[bi.grp].n_ck;
-            }
-            const int P = kGrouped ? a.groups[bi.grp].P : a.P;
-            const uint32_t gA = feed_groups(a, min(kTile, P - w.ti * kTile));
-            const uint32_t gB = feed_groups(a, min(kTile, P - w.tj * kTile));
-            const uint32_t bytes = diag ? side_bytes(gA) : side_bytes(gA) + side_bytes(gB);
-            for (int st = 0; st < nst; ++st, ++g) {
-                if (static_cast<long long>(g) == a.withhold) return;  // test hook: stop feeding
-                const int slot = static_cast<int>(g % kStages);
-                if (!waitb(&ctl->empty[slot], ((g / kStages) & 1u) ^ 1u, ctl, a)) goto abort;
-                uint8_t* sb = smem + slot * kStageBytes;
-                mbar_expect_tx(&ctl->full[slot], bytes);
-                const int64_t ci = static_cast<int64_t>(w.ti) * n_ck + bi.col / kStageK + st;
-                copy_side(sb, images + ci * kFxImageBytes, mplanes + ci * kTile8Bytes, gA, &ctl->full[slot]);
-                if (!diag) {
-                    const int64_t cj = static_cast<int64_t>(w.tj) * n_ck + bi.col / kStageK + st;
-                    copy_side(sb + kSide, images + cj * kFxImageBytes, mplanes + cj * kTile8Bytes, gB, &ctl->full[slot]);
-                }
-            }
-        }
-    }
-    return;
-abort:
-    // Let the copies already issued land before the CTA's shared memory goes away.
-    for (uint32_t k = (g >= kStages ? g - kStages : 0); k < g; ++k)
-        waitb(&ctl->full[k % kStages], (k / kStages) & 1u, ctl, a, false);
-}
-
-template <bool kGrouped>
-__device__ void fx_issuer(const FxArgs& a, uint8_t* smem, FxCtl* ctl, uint32_t tmem) {
-    uint32_t g = 0, cs = 0;
-    const uint32_t V3 = tmem, V4 = tmem + 128u, V5 = tmem + 256u, V6 = tmem + 384u;
-    for (uint32_t gi = 0;; ++gi) {
-        const int it = read_item(a, ctl, gi);
+        int it = -1;
+        if (lane == 0) it = take_item(a, ctl, gi, ok);
+        it = uni(it);
+        stopped = uni(static_cast<int>(ok)) == 0;
         if (it < 0) break;
         const WorkItem w = a.items[it];
         const BlockInfo bi = a.blocks[w.blk];
-        const int nst = stages_of(bi.k, kStageK);
-        const uint32_t id = idesc_for<kGrouped>(a, w, bi);
+        const int nst = uni(stages_of(bi.k, kStageK));
+        const bool diag = uni(static_cast<int>(w.ti == w.tj)) != 0;
+        const uint8_t* images = a.images;
+        const uint8_t* mplanes = a.mplanes;
+        int64_t n_ck = a.n_ck;
+        if constexpr (kGrouped) {
+            images = a.groups[bi.grp].images;
+            mplanes = a.groups[bi.grp].mplanes;
+            n_ck = a.groups[bi.grp].n_ck;
+        }
+        const int P = kGrouped ? a.groups[bi.grp].P : a.P;
+        const uint32_t gA = uni(feed_groups(a, min(kTile, P - w.ti * kTile)));
+        const uint32_t gB = uni(feed_groups(a, min(kTile, P - w.tj * kTile)));
+        const uint32_t bytes = diag ? side_bytes(gA) : side_bytes(gA) + side_bytes(gB);
+        const int64_t ci = static_cast<int64_t>(w.ti) * n_ck + bi.col / kStageK;
+        const int64_t cj = static_cast<int64_t>(w.tj) * n_ck + bi.col / kStageK;
+        const uint8_t* imgA = uni(images + ci * kFxImageBytes);
+        const uint8_t* mA = uni(mplanes + ci * kTile8Bytes);
+        const uint8_t* imgB = uni(images + cj * kFxImageBytes);
+        const uint8_t* mB = uni(mplanes + cj * kTile8Bytes);
+        for (int st = 0; st < nst; ++st, ++g) {
+            if (static_cast<long long>(g) == a.withhold) return;  // test hook: stop feeding
+            const int slot = static_cast<int>(g % kStages);
+            if (!waitw(&ctl->empty[slot], ((g / kStages) & 1u) ^ 1u, ctl, a, lane)) {
+                stopped = true;
+                break;
+            }
+            uint8_t* sb = smem + slot * kStageBytes;
+            if (elect_one()) {
+                mbar_expect_tx(&ctl->full[slot], bytes);
+                copy_side(sb, imgA + st * kFxImageBytes, mA + st * kTile8Bytes, gA, &ctl->full[slot]);
+                if (!diag) copy_side(sb + kSide, imgB + st * kFxImageBytes, mB + st * kTile8Bytes, gB, &ctl->full[slot]);
+            }
+            __syncwarp();
+        }
+    }
+    // After an abort, let the copies already issued land before the CTA's shared memory goes away.
+    if (stopped && lane == 0)
+        for (uint32_t k = (g >= kStages ? g - kStages : 0); k < g; ++k)
+            waitb(&ctl->full[k % kStages], (k / kStages) & 1u, ctl, a, false);
+    __syncwarp();
+}
+
+// The whole of warp 1.
+template <bool kGrouped>
+__device__ void fx_issuer(const FxArgs& a, uint8_t* smem, FxCtl* ctl, uint32_t tmem_base, int lane) {
+    uint32_t g = 0, cs = 0;
+    const uint32_t tmem = uni(tmem_base);
+    const uint32_t V3 = tmem, V4 = tmem + 128u, V5 = tmem + 256u, V6 = tmem + 384u;
+    const uint64_t d0 = smem_desc(smem_u32(smem), 256, 6);  // plane t of a side: 256 t further (16-byte units)
+    for (uint32_t gi = 0;; ++gi) {
+        int it = 0;
+        if (lane == 0) it = read_item(a, ctl, gi);
+        it = uni(it);
+        if (it < 0) break;
+        const WorkItem w = a.items[it];
+        const BlockInfo bi = a.blocks[w.blk];
+        const int nst = uni(stages_of(bi.k, kStageK));
+        const uint32_t id = uni(idesc_for<kGrouped>(a, w, bi));
         // The same shape with N = 128 + n: two adjacent B planes into two adjacent weights.
         const uint32_t id2 = (id & ~(0x3Fu << 17)) | ((((id >> 17) & 0x3Fu) + 16u) << 17);
-        const bool diag = w.ti == w.tj;
+        const uint64_t b_off = uni(static_cast<int>(w.ti == w.tj)) ? 0u : kSide / 16;
         for (int st = 0; st < nst; ++st, ++g) {
             const int sseg = st % kSegStages;
             if (sseg == 0) {  // the epilogue has read the accumulators of the previous segment
-                if (!waitb(&ctl->acc_empty[0], (cs & 1u) ^ 1u, ctl, a)) goto done;
+                if (!waitw(&ctl->acc_empty[0], (cs & 1u) ^ 1u, ctl, a, lane)) goto done;
                 tc_fence_after();
             }
             const int slot = static_cast<int>(g % kStages);
-            if (!waitb(&ctl->full[slot], (g / kStages) & 1u, ctl, a)) goto done;
+            if (!waitw(&ctl->full[slot], (g / kStages) & 1u, ctl, a, lane)) goto done;
             tc_fence_after();
-            {
-                const uint32_t sa = smem_u32(smem + slot * kStageBytes);
-                const uint32_t sb = diag ? sa : sa + kSide;
-                auto dA = [&](int t) { return smem_desc(sa + static_cast<uint32_t>(t) * 4096u, 256, 6); };
-                auto dB = [&](int t) { return smem_desc(sb + static_cast<uint32_t>(t) * 4096u, 256, 6); };
+            const bool last = sseg == kSegStages - 1 || st == nst - 1;
+            if (elect_one()) {
+                const uint64_t da = d0 + static_cast<uint64_t>(slot) * (kStageBytes / 16), db = da + b_off;
+                auto dA = [&](uint64_t t) { return da + t * 256u; };
+                auto dB = [&](uint64_t t) { return db + t * 256u; };
                 const uint32_t f = sseg == 0 ? 0u : 1u;  // the first stage of a segment overwrites
                 using C = CollectorA;
                 // Planes are 4 KiB apart and V_3..V_6 128 TMEM columns apart, so an MMA of
@@ -299,18 +318,21 @@ __device__ void fx_issuer(const FxArgs& a, uint8_t* smem, FxCtl* ctl, uint32_t t
                 mma_i8(V4, dA(5), dB(8), id, 1u);
                 mma_i8(V5, dA(6), dB(8), id, 1u);
                 mma_i8(V6, dA(7), dB(8), id, 1u);
+                mma_commit(&ctl->empty[slot]);
+                if (last) mma_commit(&ctl->acc_full[0]);
             }
-            mma_commit(&ctl->empty[slot]);
-            if (sseg == kSegStages - 1 || st == nst - 1) {
-                mma_commit(&ctl->acc_full[0]);
-                ++cs;
-            }
+            __syncwarp();
+            cs += last ? 1u : 0u;
         }
     }
 done:
-    // Every MMA this thread issued completes before TMEM is released.
-    mma_commit(&ctl->drain);
-    waitb(&ctl->drain, 0u, ctl, a, false);
+    // Every MMA this warp issued completes before TMEM is released (a commit covers its own
+    // thread's MMAs: the elected lane is the same one throughout).
+    if (elect_one()) {
+        mma_commit(&ctl->drain);
+        waitb(&ctl->drain, 0u, ctl, a, false);
+    }
+    __syncwarp();
 }
 
 struct ItemOut {
@@ -545,8 +567,8 @@ f2_fx_kernel(const __grid_constant__ FxArgs a) {
     // complete: the images are ready, only the epilogue waits for the counts.
     if (warp >= kEpiWarp0) pdl_wait();
     if (warp < kEpiWarp0) {
-        if (warp == 0 && lane == 0) fx_producer<kGrouped>(a, smem, ctl);
-        if (warp == 1 && lane == 0) fx_issuer<kGrouped>(a, smem, ctl, tmem);
+        if (warp == 0) fx_producer<kGrouped>(a, smem, ctl, lane);
+        else fx_issuer<kGrouped>(a, smem, ctl, tmem, lane);
     } else {
         fx_epilogue<kGrouped>(a, ctl, tmem, warp, lane);
     }
@@ -610,102 +632,125 @@ __device__ __forceinline__ void vp_copy_region(uint8_t* dst, const uint8_t* src,
         for (int j = 0; j < n && g != 0; ++j) bulk_load(dst + j * 4096, src + j * 4096, g * 256u, bar);
 }
 
+// The whole of warp 0.
 template <bool kGrouped>
-__device__ void vp_producer(const FxArgs& a, uint8_t* smem, FxCtl* ctl) {
+__device__ void vp_producer(const FxArgs& a, uint8_t* smem, FxCtl* ctl, int lane) {
     uint32_t g = 0;
-    int u_next = atomicAdd(a.next_item, 1);
-    for (uint32_t gi = 0;; ++gi) {
+    int u_next = 0;
+    if (lane == 0) u_next = atomicAdd(a.next_item, 1);
+    bool stopped = false;
+    for (uint32_t gi = 0; !stopped; ++gi) {
         bool ok = true;
-        const int it = take_unit(a, ctl, gi, u_next, ok);
-        if (!ok) goto abort;
+        int it = -1;
+        if (lane == 0) it = take_unit(a, ctl, gi, u_next, ok);
+        it = uni(it);
+        stopped = uni(static_cast<int>(ok)) == 0;
         if (it < 0) break;
-        {
-            const WorkItem w = a.items[it];
-            const bool pair = vp_second(a, it) >= 0;
-            const BlockInfo bi = a.blocks[w.blk];
-            const int nch = stages_of(bi.k, kStageK);
-            const bool diag = w.ti == w.tj;
-            const uint8_t* mt = a.mplanes;
-            int64_t n_ck = a.n_ck;
-            if constexpr (kGrouped) {
-                mt = a.groups[bi.grp].mplanes;
-                n_ck = a.groups[bi.grp].n_ck;
+        const WorkItem w = a.items[it];
+        const bool pair = vp_second(a, it) >= 0;
+        const BlockInfo bi = a.blocks[w.blk];
+        const int nch = uni(stages_of(bi.k, kStageK));
+        const bool diag = w.ti == w.tj;
+        const uint8_t* mt = a.mplanes;
+        int64_t n_ck = a.n_ck;
+        if constexpr (kGrouped) {
+            mt = a.groups[bi.grp].mplanes;
+            n_ck = a.groups[bi.grp].n_ck;
+        }
+        // Per chunk: the valid 8-row groups of a partial side (feed_groups), else 4 KiB.
+        const int P = kGrouped ? a.groups[bi.grp].P : a.P;
+        const uint32_t gA = uni(diag ? 0u : feed_groups(a, min(kTile, P - w.ti * kTile)));
+        const uint32_t gB = uni(feed_groups(a, min(kTile, P - w.tj * kTile)));
+        const uint32_t gF = uni(pair ? feed_groups(a, min(kTile, P - (w.tj + 1) * kTile)) : 0u);
+        const int64_t chunk = bi.col / kStageK;
+        const uint8_t* si = uni(mt + (static_cast<int64_t>(w.ti) * n_ck + chunk) * kTile8Bytes);
+        const uint8_t* sj = uni(mt + (static_cast<int64_t>(w.tj) * n_ck + chunk) * kTile8Bytes);
+        const uint8_t* sf = uni(mt + (static_cast<int64_t>(w.tj + 1) * n_ck + chunk) * kTile8Bytes);
+        for (int c0 = 0; c0 < nch; c0 += kVpChunks, ++g) {
+            const int n = min(kVpChunks, nch - c0);
+            const int slot = static_cast<int>(g % kVpStages);
+            if (!waitw(&ctl->empty[slot], ((g / kVpStages) & 1u) ^ 1u, ctl, a, lane)) {
+                stopped = true;
+                break;
             }
-            // Per chunk: the valid 8-row groups of a partial side (feed_groups), else 4 KiB.
-            const int P = kGrouped ? a.groups[bi.grp].P : a.P;
-            const uint32_t gA = diag ? 0u : feed_groups(a, min(kTile, P - w.ti * kTile));
-            const uint32_t gB = feed_groups(a, min(kTile, P - w.tj * kTile));
-            const uint32_t gF = pair ? feed_groups(a, min(kTile, P - (w.tj + 1) * kTile)) : 0u;
-            for (int c0 = 0; c0 < nch; c0 += kVpChunks, ++g) {
-                const int n = min(kVpChunks, nch - c0);
-                const int slot = static_cast<int>(g % kVpStages);
-                if (!waitb(&ctl->empty[slot], ((g / kVpStages) & 1u) ^ 1u, ctl, a)) goto abort;
-                uint8_t* sa = smem + slot * kVpStageBytes;
-                unsigned long long* bar = &ctl->full[slot];
+            uint8_t* sa = smem + slot * kVpStageBytes;
+            unsigned long long* bar = &ctl->full[slot];
+            if (elect_one()) {
                 mbar_expect_tx(bar, static_cast<uint32_t>(n) * (chunk_bytes(gA) + chunk_bytes(gB) + chunk_bytes(gF)));
-                const int64_t chunk = bi.col / kStageK + c0;
-                const uint8_t* si = mt + (static_cast<int64_t>(w.ti) * n_ck + chunk) * kTile8Bytes;
-                const uint8_t* sj = mt + (static_cast<int64_t>(w.tj) * n_ck + chunk) * kTile8Bytes;
-                vp_copy_region(sa, si, gA, n, bar);
-                vp_copy_region(sa + kVpASide, sj, gB, n, bar);
-                vp_copy_region(sa + 2 * kVpASide, sj + n_ck * kTile8Bytes, gF, n, bar);
+                const int64_t o = static_cast<int64_t>(c0) * kTile8Bytes;
+                vp_copy_region(sa, si + o, gA, n, bar);
+                vp_copy_region(sa + kVpASide, sj + o, gB, n, bar);
+                vp_copy_region(sa + 2 * kVpASide, sf + o, gF, n, bar);
             }
+            __syncwarp();
         }
     }
-    return;
-abort:
-    for (uint32_t k = (g >= kVpStages ? g - kVpStages : 0); k < g; ++k)
-        waitb(&ctl->full[k % kVpStages], (k / kVpStages) & 1u, ctl, a, false);
+    if (stopped && lane == 0)
+        for (uint32_t k = (g >= kVpStages ? g - kVpStages : 0); k < g; ++k)
+            waitb(&ctl->full[k % kVpStages], (k / kVpStages) & 1u, ctl, a, false);
+    __syncwarp();
 }
 
+// The whole of warp 1.
 template <bool kGrouped>
-__device__ void vp_issuer(const FxArgs& a, uint8_t* smem, FxCtl* ctl, uint32_t tmem) {
+__device__ void vp_issuer(const FxArgs& a, uint8_t* smem, FxCtl* ctl, uint32_t tmem_base, int lane) {
     uint32_t g = 0, n_acc = 0;
+    const uint32_t tmem = uni(tmem_base);
+    const uint64_t d0 = smem_desc(smem_u32(smem), 256, 6);  // chunk j: 256 j further (16-byte units)
     for (uint32_t gi = 0;; ++gi) {
-        const int it = read_item(a, ctl, gi);
+        int it = 0;
+        if (lane == 0) it = read_item(a, ctl, gi);
+        it = uni(it);
         if (it < 0) break;
         const WorkItem w = a.items[it];
         const BlockInfo bi = a.blocks[w.blk];
-        const int nch = stages_of(bi.k, kStageK);
+        const int nch = uni(stages_of(bi.k, kStageK));
         if (nch == 0) continue;
-        const bool pair = vp_second(a, it) >= 0;
-        const uint32_t id = vp_idesc<kGrouped>(a, bi, w.tj);
-        const uint32_t idf = pair ? vp_idesc<kGrouped>(a, bi, w.tj + 1) : 0u;
-        const bool diag = w.ti == w.tj;
+        const bool pair = uni(static_cast<int>(vp_second(a, it) >= 0)) != 0;
+        const uint32_t id = uni(vp_idesc<kGrouped>(a, bi, w.tj));
+        const uint32_t idf = uni(pair ? vp_idesc<kGrouped>(a, bi, w.tj + 1) : 0u);
+        const bool diag = uni(static_cast<int>(w.ti == w.tj)) != 0;
         // One accumulator per part of at most kVpPartChunks chunks (the int32 bound).
         for (int p0 = 0; p0 < nch; p0 += kVpPartChunks) {
             const int p1 = min(nch, p0 + kVpPartChunks);
             const int b = static_cast<int>(n_acc % kVpAcc);
-            if (!waitb(&ctl->acc_empty[b], ((n_acc / kVpAcc) & 1u) ^ 1u, ctl, a)) goto done;
+            if (!waitw(&ctl->acc_empty[b], ((n_acc / kVpAcc) & 1u) ^ 1u, ctl, a, lane)) goto done;
             tc_fence_after();
             const uint32_t d = tmem + static_cast<uint32_t>(b) * kVpAccCols;
             for (int c0 = p0; c0 < p1; c0 += kVpChunks, ++g) {
                 const int slot = static_cast<int>(g % kVpStages);
-                if (!waitb(&ctl->full[slot], (g / kVpStages) & 1u, ctl, a)) goto done;
+                if (!waitw(&ctl->full[slot], (g / kVpStages) & 1u, ctl, a, lane)) goto done;
                 tc_fence_after();
-                const uint32_t sa = smem_u32(smem + slot * kVpStageBytes);
-                const uint32_t sb = sa + kVpASide;
                 const int n = min(kVpChunks, nch - c0);
-                for (int j = 0; j < n; ++j) {
-                    const uint32_t bj = sb + static_cast<uint32_t>(j) * 4096u;
-                    const uint64_t dA = smem_desc(diag ? bj : sa + static_cast<uint32_t>(j) * 4096u, 256, 6);
-                    const uint32_t f = (c0 + j) > p0 ? 1u : 0u;
-                    if (pair) {
-                        mma_i8_c<CollectorA::kFill>(d, dA, smem_desc(bj, 256, 6), id, f);
-                        mma_i8_c<CollectorA::kLastUse>(d + kTile, dA, smem_desc(bj + kVpASide, 256, 6), idf, f);
-                    } else {
-                        mma_i8(d, dA, smem_desc(bj, 256, 6), id, f);
+                if (elect_one()) {
+                    const uint64_t da = d0 + static_cast<uint64_t>(slot) * (kVpStageBytes / 16), db = da + kVpASide / 16;
+#pragma unroll
+                    for (int j = 0; j < kVpChunks; ++j) {
+                        if (j >= n) break;
+                        const uint64_t bj = db + static_cast<uint64_t>(j) * 256u;
+                        const uint64_t aj = diag ? bj : da + static_cast<uint64_t>(j) * 256u;
+                        const uint32_t f = (c0 + j) > p0 ? 1u : 0u;
+                        if (pair) {
+                            mma_i8_c<CollectorA::kFill>(d, aj, bj, id, f);
+                            mma_i8_c<CollectorA::kLastUse>(d + kTile, aj, bj + kVpASide / 16, idf, f);
+                        } else {
+                            mma_i8(d, aj, bj, id, f);
+                        }
                     }
+                    mma_commit(&ctl->empty[slot]);
+                    if (c0 + kVpChunks >= p1) mma_commit(&ctl->acc_full[b]);
                 }
-                mma_commit(&ctl->empty[slot]);
+                __syncwarp();
             }
-            mma_commit(&ctl->acc_full[b]);
             ++n_acc;
         }
     }
 done:
-    mma_commit(&ctl->drain);
-    waitb(&ctl->drain, 0u, ctl, a, false);
+    if (elect_one()) {
+        mma_commit(&ctl->drain);
+        waitb(&ctl->drain, 0u, ctl, a, false);
+    }
+    __syncwarp();
 }
 
 // Warp (quarter q, half h): TMEM lanes 32q.., columns 128h.. of the accumulator, i.e. the
@@ -785,8 +830,8 @@ __global__ void __launch_bounds__(kVpThreads, 1) vpair_fx_kernel(const __grid_co
     pdl_wait();  // the decode's M tiles
     pdl_trigger();
     if (warp < 2) {
-        if (warp == 0 && lane == 0) vp_producer<kGrouped>(a, smem, ctl);
-        if (warp == 1 && lane == 0) vp_issuer<kGrouped>(a, smem, ctl, tmem);
+        if (warp == 0) vp_producer<kGrouped>(a, smem, ctl, lane);
+        else vp_issuer<kGrouped>(a, smem, ctl, tmem, lane);
     } else {
         vp_epilogue(a, ctl, tmem, warp, lane);
     }

@@ -88,21 +88,16 @@ __device__ __forceinline__ bool waitb(unsigned long long* b, uint32_t parity, Fx
     return wait_bounded(b, parity, &ctl->abort, a.err, a.timeout_ns, honour_abort);
 }
 
+__device__ __forceinline__ bool waitw(unsigned long long* b, uint32_t parity, FxsCtl* ctl, const FxsArgs& a, int lane) {
+    return wait_warp(b, parity, &ctl->abort, a.err, a.timeout_ns, lane);
+}
+
 template <bool kGrouped>
 __device__ __forceinline__ int pops_of(const FxsArgs& a, const BlockInfo& bi) {
     return kGrouped ? bi.P : a.P;
 }
 
 __device__ __forceinline__ int chunks_of(const BlockInfo& bi) { return (bi.k + 31) / 32; }
-
-// The next item out of the ring, false when the work or the CTA has ended.
-__device__ __forceinline__ bool read_item(const FxsArgs& a, FxsCtl* ctl, uint32_t gi, BlockInfo& bi) {
-    const int slot = static_cast<int>(gi % kItemRing);
-    if (!waitb(&ctl->item_full[slot], (gi / kItemRing) & 1u, ctl, a)) return false;
-    bi = ctl->item[slot];
-    mbar_arrive(&ctl->item_empty[slot]);
-    return bi.k >= 0;
-}
 
 // Which accumulator slots the items use, in the issuer's and the epilogue's step: a plane of
 // up to 32 rows takes one 256-column slot, alternating; a longer one takes both. uses[s]
@@ -118,96 +113,130 @@ struct AccRing {
     }
 };
 
+// The whole of warp 0.
 template <bool kGrouped>
-__device__ void fxs_producer(const FxsArgs& a, uint8_t* smem, FxsCtl* ctl) {
+__device__ void fxs_producer(const FxsArgs& a, uint8_t* smem, FxsCtl* ctl, int lane) {
     uint32_t g = 0;
     // Two claims ahead: the counter's answer and the item's record arrive while earlier
-    // items stream.
-    int it = atomicAdd(a.next, 1);
+    // items stream (lane 0 holds them).
+    int it = a.n_work;
     BlockInfo cur{}, nxt{};
     cur.k = nxt.k = -1;
-    if (it < a.n_work) cur = a.work[it];
-    it = atomicAdd(a.next, 1);
-    for (uint32_t gi = 0;; ++gi) {
+    if (lane == 0) {
+        it = atomicAdd(a.next, 1);
+        if (it < a.n_work) cur = a.work[it];
+        it = atomicAdd(a.next, 1);
+    }
+    bool stopped = false;
+    for (uint32_t gi = 0; !stopped; ++gi) {
         const int slot = static_cast<int>(gi % kItemRing);
-        if (!waitb(&ctl->item_empty[slot], ((gi / kItemRing) & 1u) ^ 1u, ctl, a)) goto abort;
-        ctl->item[slot] = cur;
-        mbar_arrive(&ctl->item_full[slot]);
-        if (cur.k < 0) return;
+        if (!waitw(&ctl->item_empty[slot], ((gi / kItemRing) & 1u) ^ 1u, ctl, a, lane)) {
+            stopped = true;
+            break;
+        }
+        if (lane == 0) {
+            ctl->item[slot] = cur;
+            mbar_arrive(&ctl->item_full[slot]);
+        }
+        const int k = uni(cur.k);
+        if (k < 0) return;
         nxt.k = -1;
-        if (it < a.n_work) {
+        if (lane == 0 && it < a.n_work) {
             nxt = a.work[it];
             it = atomicAdd(a.next, 1);
         }
-        {
-            const int R = fxs_rows(pops_of<kGrouped>(a, cur));
-            const uint32_t chunk = static_cast<uint32_t>(kFxsPlanes * 32 * R);
-            const int per = 128 / R;
-            const uint8_t* src = (kGrouped ? a.groups[cur.grp].images : a.images) + cur.col / 32 * chunk;
-            const int nch = chunks_of(cur);
-            for (int p0 = 0; p0 < nch; p0 += kSegChunks) {
-                const int p1 = min(nch, p0 + kSegChunks);
-                for (int c0 = p0; c0 < p1; c0 += per, ++g) {
-                    if (static_cast<long long>(g) == a.withhold) return;  // test hook: stop feeding
-                    const int st = static_cast<int>(g % kStages);
-                    if (!waitb(&ctl->empty[st], ((g / kStages) & 1u) ^ 1u, ctl, a)) goto abort;
-                    const uint32_t bytes = static_cast<uint32_t>(min(per, p1 - c0)) * chunk;
+        const int grp = uni(cur.grp);
+        const int R = uni(fxs_rows(kGrouped ? uni(cur.P) : a.P));
+        const uint32_t chunk = static_cast<uint32_t>(kFxsPlanes * 32 * R);
+        const int per = 128 / R;
+        const uint8_t* src = uni((kGrouped ? a.groups[grp].images : a.images) + uni(cur.col) / 32 * chunk);
+        const int nch = (k + 31) / 32;
+        for (int p0 = 0; p0 < nch && !stopped; p0 += kSegChunks) {
+            const int p1 = min(nch, p0 + kSegChunks);
+            for (int c0 = p0; c0 < p1; c0 += per, ++g) {
+                if (static_cast<long long>(g) == a.withhold) return;  // test hook: stop feeding
+                const int st = static_cast<int>(g % kStages);
+                if (!waitw(&ctl->empty[st], ((g / kStages) & 1u) ^ 1u, ctl, a, lane)) {
+                    stopped = true;
+                    break;
+                }
+                const uint32_t bytes = static_cast<uint32_t>(min(per, p1 - c0)) * chunk;
+                if (elect_one()) {
                     mbar_expect_tx(&ctl->full[st], bytes);
                     bulk_load(smem + st * kStageBytes, src + static_cast<int64_t>(c0) * chunk, bytes, &ctl->full[st]);
                 }
+                __syncwarp();
             }
         }
         cur = nxt;
     }
-abort:
-    // Let the copies already issued land before the CTA's shared memory goes away.
-    for (uint32_t k = (g >= kStages ? g - kStages : 0); k < g; ++k)
-        waitb(&ctl->full[k % kStages], (k / kStages) & 1u, ctl, a, false);
+    // After an abort, let the copies already issued land before the CTA's shared memory goes away.
+    if (lane == 0)
+        for (uint32_t k = (g >= kStages ? g - kStages : 0); k < g; ++k)
+            waitb(&ctl->full[k % kStages], (k / kStages) & 1u, ctl, a, false);
+    __syncwarp();
 }
 
+// The whole of warp 1.
 template <bool kGrouped>
-__device__ void fxs_issuer(const FxsArgs& a, uint8_t* smem, FxsCtl* ctl, uint32_t tmem) {
+__device__ void fxs_issuer(const FxsArgs& a, uint8_t* smem, FxsCtl* ctl, uint32_t tmem_base, int lane) {
     uint32_t g = 0;
+    const uint32_t tmem = uni(tmem_base);
+    const uint64_t d0 = smem_desc(smem_u32(smem), 256, 6);
     AccRing acc;
-    BlockInfo bi;
-    for (uint32_t gi = 0; read_item(a, ctl, gi, bi); ++gi) {
-        const int R = fxs_rows(pops_of<kGrouped>(a, bi));
-        const uint32_t plane = static_cast<uint32_t>(32 * R);
-        const int per = 128 / R;
-        // D = s32, A = B = s8, K-major, N = 4R, M = 128.
-        const uint32_t id = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(4 * R) >> 3 << 17) | (8u << 24);
-        const int nch = chunks_of(bi);
-        for (int p0 = 0; p0 < nch; p0 += kSegChunks) {
-            const int p1 = min(nch, p0 + kSegChunks);
-            const int s = acc.slot(R);
-            if (!waitb(&ctl->acc_empty[s], (acc.uses[s] & 1u) ^ 1u, ctl, a)) goto done;
-            ++acc.uses[s];
-            if (R > 32) {
-                if (!waitb(&ctl->acc_empty[1], (acc.uses[1] & 1u) ^ 1u, ctl, a)) goto done;
-                ++acc.uses[1];
-            }
-            tc_fence_after();
-            const uint32_t d1 = tmem + static_cast<uint32_t>(s) * 256u, d2 = d1 + static_cast<uint32_t>(4 * R);
-            for (int c0 = p0; c0 < p1; c0 += per, ++g) {
-                const int st = static_cast<int>(g % kStages);
-                if (!waitb(&ctl->full[st], (g / kStages) & 1u, ctl, a)) goto done;
-                tc_fence_after();
-                uint32_t sa = smem_u32(smem + st * kStageBytes);
-                const int n = min(per, p1 - c0);
-                for (int j = 0; j < n; ++j, sa += kFxsPlanes * plane) {
-                    const uint32_t f = c0 + j > p0 ? 1u : 0u;
-                    mma_i8(d1, smem_desc(sa + 2 * plane, 256, 6), smem_desc(sa, 256, 6), id, f);
-                    mma_i8(d2, smem_desc(sa + 4 * plane, 256, 6), smem_desc(sa + 5 * plane, 256, 6), id, f);
+    for (uint32_t gi = 0;; ++gi) {
+        const int slot = static_cast<int>(gi % kItemRing);
+        if (!waitw(&ctl->item_full[slot], (gi / kItemRing) & 1u, ctl, a, lane)) goto done;
+        {
+            const BlockInfo bi = ctl->item[slot];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl->item_empty[slot]);
+            const int k = uni(bi.k);
+            if (k < 0) break;
+            const int R = uni(fxs_rows(pops_of<kGrouped>(a, bi)));
+            const uint64_t plane = static_cast<uint64_t>(2 * R);  // 32 R bytes, in 16-byte units
+            const int per = 128 / R;
+            // D = s32, A = B = s8, K-major, N = 4R, M = 128.
+            const uint32_t id = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(4 * R) >> 3 << 17) | (8u << 24);
+            const int nch = (k + 31) / 32;
+            for (int p0 = 0; p0 < nch; p0 += kSegChunks) {
+                const int p1 = min(nch, p0 + kSegChunks);
+                const int s = acc.slot(R);
+                if (!waitw(&ctl->acc_empty[s], (acc.uses[s] & 1u) ^ 1u, ctl, a, lane)) goto done;
+                ++acc.uses[s];
+                if (R > 32) {
+                    if (!waitw(&ctl->acc_empty[1], (acc.uses[1] & 1u) ^ 1u, ctl, a, lane)) goto done;
+                    ++acc.uses[1];
                 }
-                mma_commit(&ctl->empty[st]);
+                tc_fence_after();
+                const uint32_t d1 = tmem + static_cast<uint32_t>(s) * 256u, d2 = d1 + static_cast<uint32_t>(4 * R);
+                for (int c0 = p0; c0 < p1; c0 += per, ++g) {
+                    const int st = static_cast<int>(g % kStages);
+                    if (!waitw(&ctl->full[st], (g / kStages) & 1u, ctl, a, lane)) goto done;
+                    tc_fence_after();
+                    const int n = min(per, p1 - c0);
+                    if (elect_one()) {
+                        uint64_t da = d0 + static_cast<uint64_t>(st) * (kStageBytes / 16);
+                        for (int j = 0; j < n; ++j, da += kFxsPlanes * plane) {
+                            const uint32_t f = c0 + j > p0 ? 1u : 0u;
+                            mma_i8(d1, da + 2 * plane, da, id, f);
+                            mma_i8(d2, da + 4 * plane, da + 5 * plane, id, f);
+                        }
+                        mma_commit(&ctl->empty[st]);
+                        if (c0 + per >= p1) mma_commit(&ctl->acc_full[s]);
+                    }
+                    __syncwarp();
+                }
             }
-            mma_commit(&ctl->acc_full[s]);
         }
     }
 done:
-    // Every MMA this thread issued completes before TMEM is released.
-    mma_commit(&ctl->drain);
-    waitb(&ctl->drain, 0u, ctl, a, false);
+    // Every MMA this warp issued completes before TMEM is released.
+    if (elect_one()) {
+        mma_commit(&ctl->drain);
+        waitb(&ctl->drain, 0u, ctl, a, false);
+    }
+    __syncwarp();
 }
 
 // A barrier of the eight epilogue warps that also tells whether any of them has seen a wait
@@ -365,8 +394,8 @@ __global__ void __launch_bounds__(kThreads, 1) f2_fxs_kernel(const __grid_consta
     const uint32_t tmem = ctl->tmem_base;
     pdl_wait();  // the decode's images
     if (warp < 2) {
-        if (warp == 0 && lane == 0) fxs_producer<kGrouped>(a, smem, ctl);
-        if (warp == 1 && lane == 0) fxs_issuer<kGrouped>(a, smem, ctl, tmem);
+        if (warp == 0) fxs_producer<kGrouped>(a, smem, ctl, lane);
+        else fxs_issuer<kGrouped>(a, smem, ctl, tmem, lane);
     } else {
         fxs_epilogue<kGrouped>(a, ctl, tmem, t_hi, t_lo, s_vp, warp, lane);
     }

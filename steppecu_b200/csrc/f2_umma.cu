@@ -113,6 +113,10 @@ __device__ __forceinline__ bool wait_bounded(unsigned long long* b, uint32_t par
     return ptx::wait_bounded(b, parity, &ctl->abort, err, kTimeoutNs, honour_abort);
 }
 
+__device__ __forceinline__ bool waitw(unsigned long long* b, uint32_t parity, SmemCtl* ctl, const UmmaArgs& a, int lane) {
+    return wait_warp(b, parity, &ctl->abort, a.err, kTimeoutNs, lane);
+}
+
 // ---- roles -------------------------------------------------------------------------------
 
 __device__ __forceinline__ int stages_of(int k) { return (k + kStageK - 1) / kStageK; }
@@ -143,117 +147,122 @@ __device__ __forceinline__ int read_item(const UmmaArgs& a, SmemCtl* ctl, uint32
     return it;
 }
 
+// The whole of warp 0.
 template <bool kGrouped>
-__device__ void producer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl) {
+__device__ void producer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, int lane) {
     uint32_t g = 0;
-    for (uint32_t gi = 0;; ++gi) {
+    bool stopped = false;
+    for (uint32_t gi = 0; !stopped; ++gi) {
         bool ok = true;
-        const int it = take_item(a, ctl, gi, ok);
-        if (!ok) goto abort;
+        int it = -1;
+        if (lane == 0) it = take_item(a, ctl, gi, ok);
+        it = uni(it);
+        stopped = uni(static_cast<int>(ok)) == 0;
         if (it < 0) break;
         const WorkItem w = a.items[it];
         const BlockInfo bi = a.blocks[w.blk];
-        const int nst = stages_of(bi.k);
-        const bool diag = w.ti == w.tj;
+        const int nst = uni(stages_of(bi.k));
+        const bool diag = uni(static_cast<int>(w.ti == w.tj)) != 0;
         const uint8_t* images = a.images;
         int64_t n_ck = a.n_ck;
         if constexpr (kGrouped) {
             images = a.groups[bi.grp].images;
             n_ck = a.groups[bi.grp].n_ck;
         }
+        const int64_t chunk = bi.col / kStageK;
+        const uint8_t* imgA = uni(images + (static_cast<int64_t>(w.ti) * n_ck + chunk) * kSideBytes);
+        const uint8_t* imgB = uni(images + (static_cast<int64_t>(w.tj) * n_ck + chunk) * kSideBytes);
         for (int st = 0; st < nst; ++st, ++g) {
             const int slot = static_cast<int>(g % kStages);
-            const uint32_t ph = (g / kStages) & 1u;
-            if (!wait_bounded(&ctl->empty[slot], ph ^ 1u, ctl, a.err)) goto abort;
-            {
-                uint8_t* sb = smem + slot * kStageBytes;
-                mbar_expect_tx(&ctl->full[slot], diag ? kSideBytes : kStageBytes);
-                const int64_t chunk = bi.col / kStageK + st;
-                const int64_t ta = static_cast<int64_t>(w.ti) * n_ck + chunk;
-                bulk_load(sb, images + ta * kSideBytes, kSideBytes, &ctl->full[slot]);
-                if (!diag) {
-                    const int64_t tb = static_cast<int64_t>(w.tj) * n_ck + chunk;
-                    bulk_load(sb + kSideBytes, images + tb * kSideBytes, kSideBytes, &ctl->full[slot]);
-                }
+            if (!waitw(&ctl->empty[slot], ((g / kStages) & 1u) ^ 1u, ctl, a, lane)) {
+                stopped = true;
+                break;
             }
+            uint8_t* sb = smem + slot * kStageBytes;
+            if (elect_one()) {
+                mbar_expect_tx(&ctl->full[slot], diag ? kSideBytes : kStageBytes);
+                bulk_load(sb, imgA + static_cast<int64_t>(st) * kSideBytes, kSideBytes, &ctl->full[slot]);
+                if (!diag) bulk_load(sb + kSideBytes, imgB + static_cast<int64_t>(st) * kSideBytes, kSideBytes, &ctl->full[slot]);
+            }
+            __syncwarp();
         }
     }
-    return;
-abort:
-    // Let the copies already issued land before the CTA's shared memory goes away.
-    for (uint32_t k = (g >= kStages ? g - kStages : 0); k < g; ++k)
-        wait_bounded(&ctl->full[k % kStages], (k / kStages) & 1u, ctl, a.err, false);
+    // After an abort, let the copies already issued land before the CTA's shared memory goes away.
+    if (stopped && lane == 0)
+        for (uint32_t k = (g >= kStages ? g - kStages : 0); k < g; ++k)
+            wait_bounded(&ctl->full[k % kStages], (k / kStages) & 1u, ctl, a.err, false);
+    __syncwarp();
 }
 
+// The whole of warp 1.
 template <int kChunkStages>
-__device__ void mma_issuer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, uint32_t tmem) {
+__device__ void mma_issuer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, uint32_t tmem_base, int lane) {
     uint32_t g = 0, cs = 0, is = 0;
+    const uint32_t tmem = uni(tmem_base);
+    const uint32_t d_vp = tmem + kVpCol;
+    const uint64_t d16 = smem_desc(smem_u32(smem), 512, 4), d8 = smem_desc(smem_u32(smem) + kPlanes * kTile16, 256, 6);
     for (uint32_t gi = 0;; ++gi) {
-        const int it = read_item(a, ctl, gi);
+        int it = 0;
+        if (lane == 0) it = read_item(a, ctl, gi);
+        it = uni(it);
         if (it < 0) break;
         const WorkItem w = a.items[it];
         const BlockInfo bi = a.blocks[w.blk];
-        const int nst = stages_of(bi.k);
+        const int nst = uni(stages_of(bi.k));
         if (nst == 0) continue;
-        const bool diag = w.ti == w.tj;
-        {
-            const uint32_t d_vp = tmem + kVpCol;
-            for (int st = 0; st < nst; ++st, ++g) {
-                const int sc = st % kChunkStages;  // stage within the chunk
-                const int nb = static_cast<int>(cs % kNumBufs);
-                if (sc == 0) {
-                    if (!wait_bounded(&ctl->acc_empty[nb], ((cs / kNumBufs) & 1u) ^ 1u, ctl, a.err)) goto done;
-                    tc_fence_after();
-                }
-                const uint32_t d_num = tmem + static_cast<uint32_t>(nb) * 128u;
-                const int slot = static_cast<int>(g % kStages);
-                if (!wait_bounded(&ctl->full[slot], (g / kStages) & 1u, ctl, a.err)) goto done;
+        const uint64_t b_off = uni(static_cast<int>(w.ti == w.tj)) ? 0u : kSideBytes / 16;
+        for (int st = 0; st < nst; ++st, ++g) {
+            const int sc = st % kChunkStages;  // stage within the chunk
+            const int nb = static_cast<int>(cs % kNumBufs);
+            if (sc == 0) {
+                if (!waitw(&ctl->acc_empty[nb], ((cs / kNumBufs) & 1u) ^ 1u, ctl, a, lane)) goto done;
                 tc_fence_after();
-                const uint32_t sa = smem_u32(smem + slot * kStageBytes);
-                const uint32_t sb = diag ? sa : sa + kSideBytes;
-#pragma unroll
-                for (int k = 0; k < kStageK / 16; ++k) {
-                    const uint32_t ko = static_cast<uint32_t>(k) * 32u;  // 16 elements x 2 bytes
-                    const uint64_t aPh = smem_desc(sa + 0 * kTile16 + ko, 512, 4);
-                    const uint64_t aPl = smem_desc(sa + 1 * kTile16 + ko, 512, 4);
-                    const uint64_t aAh = smem_desc(sa + 2 * kTile16 + ko, 512, 4);
-                    const uint64_t aAl = smem_desc(sa + 3 * kTile16 + ko, 512, 4);
-                    const uint64_t aM = smem_desc(sa + 4 * kTile16 + ko, 512, 4);
-                    const uint64_t bPh = smem_desc(sb + 0 * kTile16 + ko, 512, 4);
-                    const uint64_t bPl = smem_desc(sb + 1 * kTile16 + ko, 512, 4);
-                    const uint64_t bAh = smem_desc(sb + 2 * kTile16 + ko, 512, 4);
-                    const uint64_t bAl = smem_desc(sb + 3 * kTile16 + ko, 512, 4);
-                    const uint64_t bM = smem_desc(sb + 4 * kTile16 + ko, 512, 4);
-                    const uint32_t first = (sc == 0 && k == 0) ? 0u : 1u;
-                    // Large terms first and interleaved in sign, the lo corrections last.
-                    mma_f16(d_num, aAh, bM, a.idesc_am, first);
-                    mma_f16(d_num, aPh, bPh, a.idesc_pp, 1u);
-                    mma_f16(d_num, aM, bAh, a.idesc_am, 1u);
-                    mma_f16(d_num, aPh, bPl, a.idesc_pp, 1u);
-                    mma_f16(d_num, aPl, bPh, a.idesc_pp, 1u);
-                    mma_f16(d_num, aAl, bM, a.idesc_am, 1u);
-                    mma_f16(d_num, aM, bAl, a.idesc_am, 1u);
-                }
-                if (st == 0) {  // the previous tile's vpair has been read
-                    if (!wait_bounded(&ctl->vp_empty, (is & 1u) ^ 1u, ctl, a.err)) goto done;
-                    tc_fence_after();
-                }
-                mma_i8(d_vp, smem_desc(sa + kPlanes * kTile16, 256, 6), smem_desc(sb + kPlanes * kTile16, 256, 6),
-                       a.idesc_i8, st > 0 ? 1u : 0u);
-                mma_commit(&ctl->empty[slot]);
-                if (sc == kChunkStages - 1 || st == nst - 1) {
-                    mma_commit(&ctl->acc_full[nb]);
-                    ++cs;
-                }
             }
-            mma_commit(&ctl->vp_full);
-            ++is;
+            if (st == 0) {  // the previous tile's vpair has been read
+                if (!waitw(&ctl->vp_empty, (is & 1u) ^ 1u, ctl, a, lane)) goto done;
+                tc_fence_after();
+            }
+            const uint32_t d_num = tmem + static_cast<uint32_t>(nb) * 128u;
+            const int slot = static_cast<int>(g % kStages);
+            if (!waitw(&ctl->full[slot], (g / kStages) & 1u, ctl, a, lane)) goto done;
+            tc_fence_after();
+            const bool end = sc == kChunkStages - 1 || st == nst - 1;
+            if (elect_one()) {
+                const uint64_t so = static_cast<uint64_t>(slot) * (kStageBytes / 16);
+                const uint64_t da = d16 + so, db = da + b_off;
+#pragma unroll
+                for (uint64_t k = 0; k < kStageK / 16; ++k) {
+                    // Plane p, k-step k (16 elements of 2 bytes): 8 KiB p + 32 k bytes further.
+                    auto A = [&](uint64_t p) { return da + p * (kTile16 / 16) + 2 * k; };
+                    auto B = [&](uint64_t p) { return db + p * (kTile16 / 16) + 2 * k; };
+                    const uint32_t first = (sc == 0 && k == 0) ? 0u : 1u;
+                    // Planes: 0 Ph, 1 Pl, 2 Ah, 3 Al, 4 M. Large terms first and interleaved in
+                    // sign, the lo corrections last.
+                    mma_f16(d_num, A(2), B(4), a.idesc_am, first);
+                    mma_f16(d_num, A(0), B(0), a.idesc_pp, 1u);
+                    mma_f16(d_num, A(4), B(2), a.idesc_am, 1u);
+                    mma_f16(d_num, A(0), B(1), a.idesc_pp, 1u);
+                    mma_f16(d_num, A(1), B(0), a.idesc_pp, 1u);
+                    mma_f16(d_num, A(3), B(4), a.idesc_am, 1u);
+                    mma_f16(d_num, A(4), B(3), a.idesc_am, 1u);
+                }
+                mma_i8(d_vp, d8 + so, d8 + so + b_off, a.idesc_i8, st > 0 ? 1u : 0u);
+                mma_commit(&ctl->empty[slot]);
+                if (end) mma_commit(&ctl->acc_full[nb]);
+                if (st == nst - 1) mma_commit(&ctl->vp_full);
+            }
+            __syncwarp();
+            cs += end ? 1u : 0u;
         }
+        ++is;
     }
 done:
-    // Every MMA this thread issued completes before TMEM is released.
-    mma_commit(&ctl->drain);
-    wait_bounded(&ctl->drain, 0u, ctl, a.err, false);
+    // Every MMA this warp issued completes before TMEM is released.
+    if (elect_one()) {
+        mma_commit(&ctl->drain);
+        wait_bounded(&ctl->drain, 0u, ctl, a.err, false);
+    }
+    __syncwarp();
 }
 
 // The output side of a work item for this epilogue thread (row r of the tile, column
@@ -478,8 +487,8 @@ f2_umma_kernel(const __grid_constant__ UmmaArgs a) {
     const uint32_t tmem = ctl->tmem_base;
 
     if (warp < kEpiWarp0) {
-        if (warp == 0 && lane == 0) producer<kGrouped>(a, smem, ctl);
-        if (warp == 1 && lane == 0) mma_issuer<kChunkStages>(a, smem, ctl, tmem);
+        if (warp == 0) producer<kGrouped>(a, smem, ctl, lane);
+        else mma_issuer<kChunkStages>(a, smem, ctl, tmem, lane);
     } else {
         epilogue<kChunkStages, kGrouped>(a, ctl, tmem, warp, lane,
                  reinterpret_cast<double*>(smem + kStages * kStageBytes + kCtlBytes) + (warp - kEpiWarp0) * kStageDoubles);

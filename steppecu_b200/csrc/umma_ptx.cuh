@@ -70,6 +70,41 @@ __device__ __forceinline__ bool wait_bounded(unsigned long long* b, uint32_t par
     }
 }
 
+// ---- warp-uniform issue ----
+//
+// tcgen05.mma, tcgen05.commit and cp.async.bulk take their operands from uniform registers. A
+// role that runs as one lane of a divergent branch computes them in vector registers and
+// moves each over per instruction. So a whole warp runs an issuing role, every value that
+// reaches those instructions made uniform where it enters (uni), and one elected lane executes
+// them, with descriptors that differ by constants from one per slot. Against single-lane roles:
+// f2 at 100 populations x 1.15M SNPs 269 -> 254 us, at 603 ragged ones 1,341 -> 1,294; their
+// counts 133 -> 114; the split form at 300 x 400,000 832 -> 809. At 1,000 populations the tensor
+// and shared-memory pipes bound f2 and it stays where it was.
+__device__ __forceinline__ int uni(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ uint32_t uni(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ int64_t uni(int64_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+template <class T>
+__device__ __forceinline__ const T* uni(const T* p) {
+    return reinterpret_cast<const T*>(uni(static_cast<int64_t>(reinterpret_cast<uintptr_t>(p))));
+}
+
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+// wait_bounded for a whole warp: the answer is the same for every lane.
+__device__ __forceinline__ bool wait_warp(unsigned long long* b, uint32_t parity, volatile int* abort_flag, int* err,
+                                          unsigned long long timeout_ns, int lane) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
+    int ok = 1;
+    if (lane == 0) ok = wait_bounded(b, parity, abort_flag, err, timeout_ns);
+    ok = uni(ok);
+    __syncwarp();
+    return ok != 0;
+}
+
 // Plain bulk copy global -> shared, completing on an mbarrier (no tensor map, no
 // multicast): size and both addresses multiples of 16 bytes.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, unsigned long long* bar) {

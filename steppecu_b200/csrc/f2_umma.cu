@@ -147,6 +147,29 @@ __device__ __forceinline__ int read_item(const UmmaArgs& a, SmemCtl* ctl, uint32
     return it;
 }
 
+// A tile side with few populations: the 8-row groups a stage copies of it (all 16 in one copy,
+// or, up to half of them, the valid ones of each plane in six copies), and the MMA columns of
+// a column tile (its populations rounded up to 16). Rows and columns past the valid ones make
+// accumulators that nothing reads, whatever the slot held there. 300 populations leave a last
+// tile of 44, and half of their tile pairs meet it: the kernel 809 -> 744 us.
+__device__ __forceinline__ uint32_t side_groups(int rows) {
+    const uint32_t g = static_cast<uint32_t>((rows + 7) / 8);
+    return g <= 8 ? g : 16u;
+}
+__device__ __forceinline__ uint32_t side_bytes(uint32_t g) { return g == 16 ? kSideBytes : g * (kPlanes * 512u + 256u); }
+__device__ __forceinline__ void copy_side(uint8_t* dst, const uint8_t* img, uint32_t g, unsigned long long* bar) {
+    if (g == 16) {
+        bulk_load(dst, img, kSideBytes, bar);
+        return;
+    }
+#pragma unroll
+    for (uint32_t pl = 0; pl < kPlanes; ++pl) bulk_load(dst + pl * kTile16, img + pl * kTile16, g * 512u, bar);
+    bulk_load(dst + kPlanes * kTile16, img + kPlanes * kTile16, g * 256u, bar);
+}
+__device__ __forceinline__ uint32_t with_columns(uint32_t idesc, int cols) {
+    return (idesc & ~(0x3Fu << 17)) | (static_cast<uint32_t>((cols + 15) / 16 * 2) << 17);
+}
+
 // The whole of warp 0.
 template <bool kGrouped>
 __device__ void producer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, int lane) {
@@ -172,6 +195,10 @@ __device__ void producer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, int lan
         const int64_t chunk = bi.col / kStageK;
         const uint8_t* imgA = uni(images + (static_cast<int64_t>(w.ti) * n_ck + chunk) * kSideBytes);
         const uint8_t* imgB = uni(images + (static_cast<int64_t>(w.tj) * n_ck + chunk) * kSideBytes);
+        const int P = kGrouped ? a.groups[bi.grp].P : a.P;
+        const uint32_t gA = uni(side_groups(min(kTile, P - w.ti * kTile)));
+        const uint32_t gB = uni(side_groups(min(kTile, P - w.tj * kTile)));
+        const uint32_t bytes = side_bytes(gA) + (diag ? 0u : side_bytes(gB));
         for (int st = 0; st < nst; ++st, ++g) {
             const int slot = static_cast<int>(g % kStages);
             if (!waitw(&ctl->empty[slot], ((g / kStages) & 1u) ^ 1u, ctl, a, lane)) {
@@ -180,9 +207,9 @@ __device__ void producer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, int lan
             }
             uint8_t* sb = smem + slot * kStageBytes;
             if (elect_one()) {
-                mbar_expect_tx(&ctl->full[slot], diag ? kSideBytes : kStageBytes);
-                bulk_load(sb, imgA + static_cast<int64_t>(st) * kSideBytes, kSideBytes, &ctl->full[slot]);
-                if (!diag) bulk_load(sb + kSideBytes, imgB + static_cast<int64_t>(st) * kSideBytes, kSideBytes, &ctl->full[slot]);
+                mbar_expect_tx(&ctl->full[slot], bytes);
+                copy_side(sb, imgA + static_cast<int64_t>(st) * kSideBytes, gA, &ctl->full[slot]);
+                if (!diag) copy_side(sb + kSideBytes, imgB + static_cast<int64_t>(st) * kSideBytes, gB, &ctl->full[slot]);
             }
             __syncwarp();
         }
@@ -195,7 +222,7 @@ __device__ void producer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, int lan
 }
 
 // The whole of warp 1.
-template <int kChunkStages>
+template <int kChunkStages, bool kGrouped>
 __device__ void mma_issuer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, uint32_t tmem_base, int lane) {
     uint32_t g = 0, cs = 0, is = 0;
     const uint32_t tmem = uni(tmem_base);
@@ -210,6 +237,9 @@ __device__ void mma_issuer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, uint3
         const BlockInfo bi = a.blocks[w.blk];
         const int nst = uni(stages_of(bi.k));
         if (nst == 0) continue;
+        const int cols = min(kTile, (kGrouped ? a.groups[bi.grp].P : a.P) - w.tj * kTile);
+        const uint32_t id_pp = uni(with_columns(a.idesc_pp, cols)), id_am = uni(with_columns(a.idesc_am, cols)),
+                       id_i8 = uni(with_columns(a.idesc_i8, cols));
         const uint64_t b_off = uni(static_cast<int>(w.ti == w.tj)) ? 0u : kSideBytes / 16;
         for (int st = 0; st < nst; ++st, ++g) {
             const int sc = st % kChunkStages;  // stage within the chunk
@@ -238,15 +268,15 @@ __device__ void mma_issuer(const UmmaArgs& a, uint8_t* smem, SmemCtl* ctl, uint3
                     const uint32_t first = (sc == 0 && k == 0) ? 0u : 1u;
                     // Planes: 0 Ph, 1 Pl, 2 Ah, 3 Al, 4 M. Large terms first and interleaved in
                     // sign, the lo corrections last.
-                    mma_f16(d_num, A(2), B(4), a.idesc_am, first);
-                    mma_f16(d_num, A(0), B(0), a.idesc_pp, 1u);
-                    mma_f16(d_num, A(4), B(2), a.idesc_am, 1u);
-                    mma_f16(d_num, A(0), B(1), a.idesc_pp, 1u);
-                    mma_f16(d_num, A(1), B(0), a.idesc_pp, 1u);
-                    mma_f16(d_num, A(3), B(4), a.idesc_am, 1u);
-                    mma_f16(d_num, A(4), B(3), a.idesc_am, 1u);
+                    mma_f16(d_num, A(2), B(4), id_am, first);
+                    mma_f16(d_num, A(0), B(0), id_pp, 1u);
+                    mma_f16(d_num, A(4), B(2), id_am, 1u);
+                    mma_f16(d_num, A(0), B(1), id_pp, 1u);
+                    mma_f16(d_num, A(1), B(0), id_pp, 1u);
+                    mma_f16(d_num, A(3), B(4), id_am, 1u);
+                    mma_f16(d_num, A(4), B(3), id_am, 1u);
                 }
-                mma_i8(d_vp, d8 + so, d8 + so + b_off, a.idesc_i8, st > 0 ? 1u : 0u);
+                mma_i8(d_vp, d8 + so, d8 + so + b_off, id_i8, st > 0 ? 1u : 0u);
                 mma_commit(&ctl->empty[slot]);
                 if (end) mma_commit(&ctl->acc_full[nb]);
                 if (st == nst - 1) mma_commit(&ctl->vp_full);
@@ -344,6 +374,12 @@ __device__ void epilogue(const UmmaArgs& a, SmemCtl* ctl, uint32_t tmem, int war
             stamp<kGrouped>(a, o.grp, lane);
             continue;
         }
+        // Only warps whose rows and columns hold populations read the accumulators.
+        bool mine;
+        {
+            const ItemOut o = item_out<kGrouped>(a, it, r, h);
+            mine = o.i0 < o.P && o.j0 < o.P;
+        }
 #pragma unroll
         for (int c = 0; c < kCols; ++c) acc[c] = 0.0;
         const int nch = (nst + kChunkStages - 1) / kChunkStages;
@@ -362,15 +398,17 @@ __device__ void epilogue(const UmmaArgs& a, SmemCtl* ctl, uint32_t tmem, int war
             // A lone last chunk reads its buffer twice and adds zero (exact).
             const uint32_t b1 = pair ? tmem + lane_addr + static_cast<uint32_t>(nb1) * 128u + col_addr : b0;
             const float w1 = pair ? 1.0f : 0.0f;
+            if (mine) {
 #pragma unroll
-            for (int q8 = 0; q8 < kCols / 8; ++q8) {
-                uint32_t v0[8], v1[8];
-                tmem_ld8(b0 + static_cast<uint32_t>(q8) * 8u, v0);
-                tmem_ld8(b1 + static_cast<uint32_t>(q8) * 8u, v1);
-                tmem_wait_ld();
+                for (int q8 = 0; q8 < kCols / 8; ++q8) {
+                    uint32_t v0[8], v1[8];
+                    tmem_ld8(b0 + static_cast<uint32_t>(q8) * 8u, v0);
+                    tmem_ld8(b1 + static_cast<uint32_t>(q8) * 8u, v1);
+                    tmem_wait_ld();
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    acc[q8 * 8 + c] += static_cast<double>(__fmaf_rn(w1, __uint_as_float(v1[c]), __uint_as_float(v0[c])));
+                    for (int c = 0; c < 8; ++c)
+                        acc[q8 * 8 + c] += static_cast<double>(__fmaf_rn(w1, __uint_as_float(v1[c]), __uint_as_float(v0[c])));
+                }
             }
             tc_fence_before();
             __syncwarp();
@@ -396,6 +434,14 @@ __device__ void epilogue(const UmmaArgs& a, SmemCtl* ctl, uint32_t tmem, int war
         const bool diag = o.diag;
         const int64_t row_i = o.slab + i;                              // (i, j) at row_i + P*j
         const int64_t row_j0 = o.slab + static_cast<int64_t>(P) * i0;  // (j, i0 + rr) at row_j0 + P*rr + j
+        if (!mine) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl->vp_empty);
+            stamp<kGrouped>(a, o.grp, lane);
+            ++is;
+            continue;
+        }
 #pragma unroll
         for (int q8 = 0; q8 < kCols / 8; ++q8) {
             uint32_t v[8];
@@ -488,7 +534,7 @@ f2_umma_kernel(const __grid_constant__ UmmaArgs a) {
 
     if (warp < kEpiWarp0) {
         if (warp == 0) producer<kGrouped>(a, smem, ctl, lane);
-        else mma_issuer<kChunkStages>(a, smem, ctl, tmem, lane);
+        else mma_issuer<kChunkStages, kGrouped>(a, smem, ctl, tmem, lane);
     } else {
         epilogue<kChunkStages, kGrouped>(a, ctl, tmem, warp, lane,
                  reinterpret_cast<double*>(smem + kStages * kStageBytes + kCtlBytes) + (warp - kEpiWarp0) * kStageDoubles);

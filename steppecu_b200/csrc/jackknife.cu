@@ -21,17 +21,26 @@ struct CSum {  // Neumaier compensated sum
     __device__ double value() const { return s + c; }
 };
 
-// One CTA per 32 items (a lane each, so every load is 256 contiguous bytes); its 16 warps
+// One CTA per 32 items (a lane each, so every load is 256 contiguous bytes); its 32 warps
 // take the blocks round robin, and each sum is combined over the warps through shared
 // memory, the compensations included. A thread per item walked all blocks alone: 40 CTAs and
-// a serial chain of compensated adds and divisions for 5,000 items x 714 blocks, 860 us
-// against 176 us. What depends on the block alone (its weight, n / bl and the root) is computed
-// once per warp and block, one block per lane, and shuffled.
-constexpr int kJkWarps = 16;
+// a serial chain of compensated adds and divisions for 5,000 items x 714 blocks, 860 us; 16
+// warps took 176 us, 144 us now. What depends on the block alone (its weight, n / bl, the root and
+// the reciprocals of what the items divide by) is computed once per warp and block, one block
+// per lane, and shuffled; an item's quotient is the product with the reciprocal and one
+// correction by the exact remainder (Markstein's division, 1990: with a reciprocal rounded to
+// nearest the corrected quotient is the rounded one for all but extreme exponents).
+constexpr int kJkWarps = 32;
 
 struct JkBlock {
-    double bl, rel, h, root;  // bl, bl / n, n / bl, sqrt(n / bl - 1)
+    double bl, rel, w, rw;   // bl, bl / n, 1 - bl / n, 1 / w
+    double h, root, rroot;   // n / bl, sqrt(n / bl - 1), 1 / root
 };
+
+__device__ __forceinline__ double jk_div(double a, double b, double rb) {
+    const double q = a * rb;
+    return fma(fma(-q, b, a), rb, q);
+}
 
 __device__ __forceinline__ double jk_total(CSum v, double (*s_part)[kJkWarps][32], int warp, int lane) {
     __syncthreads();  // the previous total has been read
@@ -39,7 +48,7 @@ __device__ __forceinline__ double jk_total(CSum v, double (*s_part)[kJkWarps][32
     s_part[1][warp][lane] = v.c;
     __syncthreads();
     CSum t;
-#pragma unroll
+#pragma unroll 4
     for (int w = 0; w < kJkWarps; ++w) {
         t.add(s_part[0][w][lane]);
         t.add(s_part[1][w][lane]);
@@ -52,14 +61,17 @@ template <bool kRoot, class F>
 __device__ __forceinline__ void jk_blocks(const double* __restrict__ x, const int32_t* __restrict__ bl, int64_t m, int nb,
                                           double n, int64_t k, bool real, int warp, int lane, F&& f) {
     for (int b0 = warp; b0 < nb; b0 += 32 * kJkWarps) {
-        JkBlock mine{1.0, 0.0, 0.0, 0.0};
+        JkBlock mine{1.0, 0.0, 1.0, 1.0, 0.0, 0.0, 0.0};
         const int bm = b0 + lane * kJkWarps;
         if (bm < nb) {
             mine.bl = static_cast<double>(bl[bm]);
             mine.rel = mine.bl / n;
+            mine.w = 1.0 - mine.rel;
+            mine.rw = 1.0 / mine.w;
             if constexpr (kRoot) {
                 mine.h = n / mine.bl;
                 mine.root = sqrt(mine.h - 1.0);
+                mine.rroot = 1.0 / mine.root;
             }
         }
         const int cnt = min(32, (nb - b0 + kJkWarps - 1) / kJkWarps);
@@ -68,9 +80,12 @@ __device__ __forceinline__ void jk_blocks(const double* __restrict__ x, const in
             JkBlock t;
             t.bl = __shfl_sync(0xffffffffu, mine.bl, j);
             t.rel = __shfl_sync(0xffffffffu, mine.rel, j);
+            t.w = __shfl_sync(0xffffffffu, mine.w, j);
+            t.rw = __shfl_sync(0xffffffffu, mine.rw, j);
             if constexpr (kRoot) {
                 t.h = __shfl_sync(0xffffffffu, mine.h, j);
                 t.root = __shfl_sync(0xffffffffu, mine.root, j);
+                t.rroot = __shfl_sync(0xffffffffu, mine.rroot, j);
             }
             f(t, real ? x[k + m * (b0 + j * kJkWarps)] : 0.0);
         }
@@ -90,24 +105,23 @@ jackknife_kernel(const double* __restrict__ x, const int32_t* __restrict__ bl, i
     // Weighted mean of the leave-one-out values (weights 1 - bl/n).
     CSum wnum, wden, wbl;
     jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
-        const double w = 1.0 - t.rel;
-        const double loo = (tot - v * t.rel) / w;
-        wnum.add(loo * w);
-        wden.add(w);
+        const double loo = jk_div(tot - v * t.rel, t.w, t.rw);
+        wnum.add(loo * t.w);
+        wden.add(t.w);
         wbl.add(loo * t.bl);
     });
     const double totline = jk_total(wnum, s_part, warp, lane) / jk_total(wden, s_part, warp, lane);
     const double wbl_n = jk_total(wbl, s_part, warp, lane) / n;
     CSum diff;
     jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
-        diff.add(totline - (tot - v * t.rel) / (1.0 - t.rel));
+        diff.add(totline - jk_div(tot - v * t.rel, t.w, t.rw));
     });
     const double term1 = (jk_total(diff, s_part, warp, lane) / nb) * nb;
     const double e = term1 + wbl_n;
     CSum acc;
     jk_blocks<true>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
-        const double loo = (tot - v * t.rel) / (1.0 - t.rel);
-        const double xtau = (e * t.h - loo * (t.h - 1.0) - totline) / t.root;
+        const double loo = jk_div(tot - v * t.rel, t.w, t.rw);
+        const double xtau = jk_div(e * t.h - loo * (t.h - 1.0) - totline, t.root, t.rroot);
         acc.add(xtau * xtau);
     });
     const double sum = jk_total(acc, s_part, warp, lane);

@@ -21,39 +21,53 @@ struct CSum {  // Neumaier compensated sum
     __device__ double value() const { return s + c; }
 };
 
-// One CTA per 32 items (a lane each, so every load is 256 contiguous bytes); its 32 warps
+// One CTA per 32 items (a lane each, so every load is 256 contiguous bytes); its 16 warps
 // take the blocks round robin, and each sum is combined over the warps through shared
 // memory, the compensations included. A thread per item walked all blocks alone: 40 CTAs and
-// a serial chain of compensated adds and divisions for 5,000 items x 714 blocks, 860 us; 16
-// warps took 176 us, 144 us now. What depends on the block alone (its weight, n / bl, the root and
-// the reciprocals of what the items divide by) is computed once per warp and block, one block
-// per lane, and shuffled; an item's quotient is the product with the reciprocal and one
-// correction by the exact remainder (Markstein's division, 1990: with a reciprocal rounded to
-// nearest the corrected quotient is the rounded one for all but extreme exponents).
-constexpr int kJkWarps = 32;
+// a serial chain of compensated adds and divisions for 5,000 items x 714 blocks, 860 us; 87 us
+// now (32 warps: 98 us, their 157 CTAs are one to an SM and so a wave and a bit). What depends
+// on the block alone (its weight, n / bl, the root and the reciprocals of what the items divide
+// by) is computed once per warp and block, one block per lane, and shuffled; an item's quotient
+// is the product with the reciprocal and one correction by the exact remainder (Markstein's
+// division, 1990: with a reciprocal rounded to nearest the corrected quotient is the rounded
+// one for all but extreme exponents).
+constexpr int kJkWarps = 16;
 
 struct JkBlock {
     double bl, rel, w, rw;   // bl, bl / n, 1 - bl / n, 1 / w
     double h, root, rroot;   // n / bl, sqrt(n / bl - 1), 1 / root
 };
 
+using JkParts = double[2][kJkWarps][32];  // (sum, compensation) of each warp and item
+
 __device__ __forceinline__ double jk_div(double a, double b, double rb) {
     const double q = a * rb;
     return fma(fma(-q, b, a), rb, q);
 }
 
-__device__ __forceinline__ double jk_total(CSum v, double (*s_part)[kJkWarps][32], int warp, int lane) {
-    __syncthreads();  // the previous total has been read
-    s_part[0][warp][lane] = v.s;
-    s_part[1][warp][lane] = v.c;
-    __syncthreads();
-    CSum t;
-#pragma unroll 4
-    for (int w = 0; w < kJkWarps; ++w) {
-        t.add(s_part[0][w][lane]);
-        t.add(s_part[1][w][lane]);
+// N sums over the warps, in warp order, warp k adding sum k for all: every warp adding them
+// for itself filled the FP64 pipe with the same compensated additions once per warp (144 us with 32 warps, 98 us without).
+template <int N>
+__device__ __forceinline__ void jk_totals(const CSum (&v)[N], double (&tot)[N], JkParts* p, int warp, int lane) {
+    __syncthreads();  // the previous totals have been read
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        p[k][0][warp][lane] = v[k].s;
+        p[k][1][warp][lane] = v[k].c;
     }
-    return t.value();
+    __syncthreads();
+    if (warp < N) {
+        CSum t;
+#pragma unroll 4
+        for (int w = 0; w < kJkWarps; ++w) {
+            t.add(p[warp][0][w][lane]);
+            t.add(p[warp][1][w][lane]);
+        }
+        p[warp][0][0][lane] = t.value();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) tot[k] = p[k][0][0][lane];
 }
 
 // f(block, value) for every block of this warp, in block order.
@@ -95,39 +109,43 @@ __device__ __forceinline__ void jk_blocks(const double* __restrict__ x, const in
 __global__ void __launch_bounds__(32 * kJkWarps)
 jackknife_kernel(const double* __restrict__ x, const int32_t* __restrict__ bl, int64_t m, int nb, double n, double* est,
                  double* var) {
-    __shared__ double s_part[2][kJkWarps][32];
+    __shared__ JkParts parts[3];
+    double total[1], totals[3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + lane;
     const bool real = k < m;
-    CSum num;
-    jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) { num.add(v * t.bl); });
-    const double tot = jk_total(num, s_part, warp, lane) / n;
+    CSum num[1];
+    jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) { num[0].add(v * t.bl); });
+    jk_totals(num, total, parts, warp, lane);
+    const double tot = total[0] / n;
     // Weighted mean of the leave-one-out values (weights 1 - bl/n).
-    CSum wnum, wden, wbl;
+    CSum w3[3];
     jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
         const double loo = jk_div(tot - v * t.rel, t.w, t.rw);
-        wnum.add(loo * t.w);
-        wden.add(t.w);
-        wbl.add(loo * t.bl);
+        w3[0].add(loo * t.w);
+        w3[1].add(t.w);
+        w3[2].add(loo * t.bl);
     });
-    const double totline = jk_total(wnum, s_part, warp, lane) / jk_total(wden, s_part, warp, lane);
-    const double wbl_n = jk_total(wbl, s_part, warp, lane) / n;
-    CSum diff;
+    jk_totals(w3, totals, parts, warp, lane);
+    const double totline = totals[0] / totals[1];
+    const double wbl_n = totals[2] / n;
+    CSum diff[1];
     jk_blocks<false>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
-        diff.add(totline - jk_div(tot - v * t.rel, t.w, t.rw));
+        diff[0].add(totline - jk_div(tot - v * t.rel, t.w, t.rw));
     });
-    const double term1 = (jk_total(diff, s_part, warp, lane) / nb) * nb;
+    jk_totals(diff, total, parts, warp, lane);
+    const double term1 = (total[0] / nb) * nb;
     const double e = term1 + wbl_n;
-    CSum acc;
+    CSum acc[1];
     jk_blocks<true>(x, bl, m, nb, n, k, real, warp, lane, [&](const JkBlock& t, double v) {
         const double loo = jk_div(tot - v * t.rel, t.w, t.rw);
         const double xtau = jk_div(e * t.h - loo * (t.h - 1.0) - totline, t.root, t.rroot);
-        acc.add(xtau * xtau);
+        acc[0].add(xtau * xtau);
     });
-    const double sum = jk_total(acc, s_part, warp, lane);
+    jk_totals(acc, total, parts, warp, lane);
     if (real && warp == 0) {
         est[k] = e;
-        var[k] = sum / nb;
+        var[k] = total[0] / nb;
     }
 }
 

@@ -176,6 +176,7 @@ struct Plan {
     int precision = 0;
     bool detect = false;
     BlockLayout L;
+    int64_t n_max = 0;  // entries 0..n_max of rec_n, rec_nm1
     DevBuf sel, pop_off, pos, tiles, col_snp, rec_n, rec_nm1, canon, center, blocks, items, own_planes, snp_begin;
     DevBuf fold_order;  // per 64-population group, local indices largest first (null: all equal)
     DevBuf fx_table;    // FX: the term table of every (n, a2) (OperandPlanes::fx_table)
@@ -328,7 +329,7 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     upload(p->pos, pos, s);
 
     // 1/n and 1/max(n-1, 1) for every called-allele count a population can reach.
-    const int64_t n_max = 2 * max_pop + 1;
+    const int64_t n_max = p->n_max = 2 * max_pop + 1;
     std::vector<double> rn(static_cast<size_t>(n_max) + 1, 0.0), rnm1(static_cast<size_t>(n_max) + 1, 1.0);
     for (int64_t n = 1; n <= n_max; ++n) {
         rn[n] = 1.0 / static_cast<double>(n);
@@ -1519,8 +1520,8 @@ stp_status stp_snp_keep_mask(stp_ctx* ctx, const stp_geno_view* geno, const int6
             cnt.reserve(static_cast<size_t>(n_pop) * ld * 4);
             launch_decode(*p, d_rec, nullptr, nullptr, s, 0, -1, true, cnt.as<uint32_t>(), ld);
             const double total = static_cast<double>(pop_offsets[n_pop]);
-            launch_keep_mask_counts(*ctx, cnt.as<uint32_t>(), ld, n_pop, M, p->rec_n.as<double>(), cols.ref.as<char>(),
-                                    cols.alt.as<char>(), cols.chrom.as<int32_t>(), *filter, total, d_keep.as<uint8_t>(),
+            launch_keep_mask_counts(*ctx, cnt.as<uint32_t>(), ld, n_pop, M, p->rec_n.as<double>(), p->n_max,
+                                    cols.ref.as<char>(), cols.alt.as<char>(), cols.chrom.as<int32_t>(), *filter, total, d_keep.as<uint8_t>(),
                                     summary ? d_sum.as<double>() : nullptr, s);
             STPF2_CUDA(cudaMemcpyAsync(keep, d_keep.ptr, static_cast<size_t>(M), cudaMemcpyDeviceToHost, s));
             if (summary)

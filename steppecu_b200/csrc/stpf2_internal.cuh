@@ -432,10 +432,10 @@ void launch_transpose_pa(Ctx& c, const uint8_t* records, uint64_t pitch, uint64_
 void launch_canonical_to_records(Ctx& c, const uint8_t* packed, uint64_t bpr, int64_t n_snp, int64_t n_ind,
                                  uint8_t* records, uint64_t pitch, cudaStream_t s);
 // extract-f2's per-SNP keep mask (filters.cu): from packed pop-major counts (ac2 | n << 16,
-// population i, SNP s at cnt[i * ld + s]; rec_n[n] = 1/n, 0 at n = 0) or from FP64 q / n [P x M] (i + P * s). out4
+// population i, SNP s at cnt[i * ld + s]; rec_n[n] = 1/n, 0 at n = 0, n up to n_max) or from FP64 q / n [P x M] (i + P * s). out4
 // (optional, device [4 * M]): pooled ref AF, pooled minor AF, missing fraction, pooled
 // allele count per SNP.
-void launch_keep_mask_counts(Ctx& c, const uint32_t* cnt, int64_t ld, int P, int64_t M, const double* rec_n,
+void launch_keep_mask_counts(Ctx& c, const uint32_t* cnt, int64_t ld, int P, int64_t M, const double* rec_n, int64_t n_max,
                              const char* ref, const char* alt, const int32_t* chrom, const stp_snp_filter& f,
                              double total_indiv, uint8_t* keep, double* out4, cudaStream_t s);
 void launch_keep_mask_qn(Ctx& c, const double* Q, const double* N, int P, int64_t M, const char* ref, const char* alt,

@@ -117,16 +117,16 @@ struct AccRing {
 template <bool kGrouped>
 __device__ void fxs_producer(const FxsArgs& a, uint8_t* smem, FxsCtl* ctl, int lane) {
     uint32_t g = 0;
-    // Two claims ahead: the counter's answer and the item's record arrive while earlier
-    // items stream (lane 0 holds them).
+    // A CTA's first item is its own number, read while the kernels before still run (the work
+    // list is older than they are); the counter deals out the rest. Its answer and the next
+    // item's record arrive while the current item streams (lane 0 holds them). Against a claim
+    // from the counter first the pass over 20 populations x 50,000 SNPs took 25.4 us, now 24.6.
     int it = a.n_work;
     BlockInfo cur{}, nxt{};
     cur.k = nxt.k = -1;
-    if (lane == 0) {
-        it = atomicAdd(a.next, 1);
-        if (it < a.n_work) cur = a.work[it];
-        it = atomicAdd(a.next, 1);
-    }
+    if (lane == 0) cur = a.work[blockIdx.x];
+    pdl_wait();  // the decode's images, and the counter
+    if (lane == 0) it = static_cast<int>(gridDim.x) + atomicAdd(a.next, 1);
     bool stopped = false;
     for (uint32_t gi = 0; !stopped; ++gi) {
         const int slot = static_cast<int>(gi % kItemRing);
@@ -143,7 +143,7 @@ __device__ void fxs_producer(const FxsArgs& a, uint8_t* smem, FxsCtl* ctl, int l
         nxt.k = -1;
         if (lane == 0 && it < a.n_work) {
             nxt = a.work[it];
-            it = atomicAdd(a.next, 1);
+            it = static_cast<int>(gridDim.x) + atomicAdd(a.next, 1);
         }
         const int grp = uni(cur.grp);
         const int R = uni(fxs_rows(kGrouped ? uni(cur.P) : a.P));
@@ -392,11 +392,15 @@ __global__ void __launch_bounds__(kThreads, 1) f2_fxs_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
-    pdl_wait();  // the decode's images
     if (warp < 2) {
-        if (warp == 0) fxs_producer<kGrouped>(a, smem, ctl, lane);
-        else fxs_issuer<kGrouped>(a, smem, ctl, tmem, lane);
+        if (warp == 0) {
+            fxs_producer<kGrouped>(a, smem, ctl, lane);
+        } else {
+            pdl_wait();
+            fxs_issuer<kGrouped>(a, smem, ctl, tmem, lane);
+        }
     } else {
+        pdl_wait();
         fxs_epilogue<kGrouped>(a, ctl, tmem, t_hi, t_lo, s_vp, warp, lane);
     }
     tc_fence_before();

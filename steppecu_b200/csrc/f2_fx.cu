@@ -37,7 +37,8 @@
 // cannot share the f2 kernel.)
 //
 //   f2_fx_kernel:   warp 0 producer (a 32 KiB image and a 4 KiB M copy per stage side, no
-//                   tensor maps, no multicast), warp 1 TMEM owner + single-thread MMA issuer, warps 2-17
+//                   tensor maps, no multicast), warp 1 TMEM owner + MMA issuer (whole warps, one
+//                   elected lane around each copy and MMA), warps 2-17
 //                   epilogue (four per TMEM lane quarter, 32 tile columns each).
 //   vpair_fx_kernel: warp 0 producer (16 KiB of A and of each column tile per stage),
 //                   warp 1 issuer, warps 2-9 epilogue (two per lane quarter, one item each).

@@ -4,7 +4,8 @@
 // stand in for the reference's ComputeBackend f2/decode virtuals (src/device/backend.hpp
 // :673-765) and its extract-f2 hot path (src/app/extract_f2_core.cpp:93-407). Host code
 // only: it validates arguments, builds the block layout and work lists, moves data and
-// launches the kernels in decode.cu, f2_simt.cu, f2_umma.cu and jackknife.cu. There is
+// launches the kernels in decode.cu, filters.cu, f2_fx.cu, f2_fxs.cu, f2_simt.cu, f2_umma.cu
+// and jackknife.cu. There is
 // no CPU fallback: without a CUDA device every entry point returns STP_NO_DEVICE.
 #include <algorithm>
 #include <thread>

@@ -63,8 +63,7 @@ void* pool_alloc(size_t& bytes, int& device) {
             void* p = v[best].p;
             bytes = v[best].bytes;
             s.held[device] -= bytes;
-            v[best] = v.back();
-            v.pop_back();
+            v.erase(v.begin() + static_cast<std::ptrdiff_t>(best));  // the rest stay in order of their release
             return p;
         }
     }
@@ -88,9 +87,18 @@ void pool_free(void* p, size_t bytes, int device) noexcept {
         cudaDeviceSynchronize() == cudaSuccess) {
         Store& s = store();
         std::lock_guard<std::mutex> lock(s.mu);
-        if (s.contexts[device] > 0 && s.held[device] + bytes <= kPoolBytes) {
+        std::vector<Block>& v = s.blocks[device];
+        if (s.contexts[device] > 0) {
+            // The blocks released longest ago make room: those of earlier calls of other sizes
+            // would otherwise fill the store and every later call allocate anew.
+            size_t old = 0;
+            while (s.held[device] + bytes > kPoolBytes) {
+                s.held[device] -= v[old].bytes;
+                cudaFree(v[old++].p);
+            }
+            v.erase(v.begin(), v.begin() + static_cast<std::ptrdiff_t>(old));
             try {
-                s.blocks[device].push_back(Block{p, bytes});
+                v.push_back(Block{p, bytes});
                 s.held[device] += bytes;
                 return;
             } catch (...) {

@@ -220,18 +220,26 @@ namespace {
 
 // Operand planes of one format (at planes_base, or the plan's own) and the tensor-core plan
 // that reads them. Padding columns must read as zero; decode only ever writes real SNP columns.
+// Both are built aside and take the place of what the plan holds only once they are complete,
+// so a failure (the images of the general form are up to 16 times the stacked ones) leaves the
+// plan as it was.
 void bind_contraction(Plan& p, OpFmt fmt, void* planes_base) {
     const size_t ob = operand_plane_bytes(fmt, std::max(p.P, 1), p.L.ld);
+    DevBuf own;
     if (!planes_base) {
-        p.own_planes.reserve(ob);
-        planes_base = p.own_planes.ptr;
+        own.reserve(ob);
+        planes_base = own.ptr;
     }
     STPF2_CUDA(cudaMemsetAsync(planes_base, 0, ob, p.ctx->stream));
-    bind_operand_planes(p.op, fmt, p.P, p.L.ld, planes_base);
-    if (p.umma) umma_plan_destroy(p.umma);
-    p.umma = nullptr;
+    OperandPlanes op = p.op;  // with the plan's term table
+    bind_operand_planes(op, fmt, p.P, p.L.ld, planes_base);
+    UmmaPlan* umma = nullptr;
     if (fmt != OpFmt::F32 && p.P > 0 && p.L.n_block > 0)
-        p.umma = umma_plan_create(*p.ctx, p.op, p.L, chunk_stages_of(p.precision));
+        umma = umma_plan_create(*p.ctx, op, p.L, chunk_stages_of(p.precision));
+    if (p.umma) umma_plan_destroy(p.umma);
+    p.umma = umma;
+    p.op = op;
+    p.own_planes = std::move(own);
 }
 
 // Validates a request and builds its plan. planes_base != nullptr borrows operand
@@ -457,6 +465,8 @@ void run_plan(Plan& p, const uint8_t* d_records, double* d_f2, double* d_vpair, 
     if (tev) STPF2_CUDA(cudaEventRecord((*tev)[1], s));
     if (p.precision == STP_PREC_FP32_SIMT)
         launch_f2_simt(c, p.items.as<WorkItem>(), p.n_items, p.blocks.as<BlockInfo>(), p.op, d_f2, d_vpair, s);
+    else if (!p.umma)
+        fail(STP_RUNTIME_ERROR, "the plan has no contraction");
     else
         launch_f2_umma(c, p.umma, d_f2, d_vpair, s, p.per_block, !tev);
     if (tev) STPF2_CUDA(cudaEventRecord((*tev)[2], s));
@@ -2176,6 +2186,10 @@ stp_status stp_plan_set_per_block_launch(stp_plan* plan, int32_t enable) {
         need(plan != nullptr, "null plan");
         Plan& p = *plan->p;
         use_device(*p.ctx);
+        if (p.graph) {  // the captured graph holds the other launch form and its operands
+            STPF2_CUDA(cudaGraphExecDestroy(p.graph));
+            p.graph = nullptr;
+        }
         // The comparison form runs the general kernels: up to kFxsMaxPops populations the
         // plan's operands change between the stacked layout and the general one.
         const OpFmt fmt = enable ? fmt_of(p.precision) : operand_fmt(p.precision, p.P, p.L);
@@ -2185,10 +2199,6 @@ stp_status stp_plan_set_per_block_launch(stp_plan* plan, int32_t enable) {
             STPF2_CUDA(cudaStreamSynchronize(p.ctx->stream));
         }
         p.per_block = enable != 0;
-        if (plan->p->graph) {  // the captured graph holds the other launch form
-            STPF2_CUDA(cudaGraphExecDestroy(plan->p->graph));
-            plan->p->graph = nullptr;
-        }
     });
 }
 

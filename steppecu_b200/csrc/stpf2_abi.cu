@@ -269,6 +269,11 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
         std::vector<int32_t> rm(p->kept.begin(), p->kept.end());
         upload(p->row_map, rm, c.stream);
     }
+    // A pitch below bytes_per_record cuts the records short: the rows must still hold every
+    // sample, in whole words, or selected samples would have no byte to be read from.
+    need(pitch >= r.geno.bytes_per_record || p->n_snp <= 0 || r.n_pop <= 0 ||
+             (pitch % 4 == 0 && pitch >= static_cast<uint64_t>((r.geno.n_ind + 3) / 4)),
+         "pitch < bytes_per_record");
     p->pitch = pitch;
     p->precision = r.precision;
     fmt_of(r.precision);  // validates the mode

@@ -187,7 +187,6 @@ struct Plan {
     double* center_ptr = nullptr;
     int64_t n_ind = 0, n_tiles = 0, n_sel_pad = 0;
     int n_items = 0;
-    bool words = true;  // records and pitch 4-byte aligned, whole rows within the pitch
     uint64_t bpr = 0;
     OperandPlanes op;
     UmmaPlan* umma = nullptr;
@@ -375,10 +374,8 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
         p->center_ptr = eb.as<double>();
     }
 
-    // The decode reads records of any pitch and alignment in place.
+    // The decode reads records of any pitch and alignment in place, and of any base on each run.
     p->bpr = r.geno.bytes_per_record;
-    p->words = pitch % 4 == 0 && pitch >= static_cast<uint64_t>((r.geno.n_ind + 3) / 4) &&
-               !(r.geno.on_device && reinterpret_cast<uintptr_t>(r.geno.records) % 4 != 0);
     if (counts_only) return p;  // decode to counts only: no operand planes, no contraction
 
     // A plan cached on the context borrows the shared planes workspace, so building another
@@ -411,16 +408,13 @@ void launch_decode(Plan& p, const uint8_t* d_records, int32_t* cnt_ac2, int32_t*
     Ctx& c = *p.ctx;
     if (p.n_snp <= 0) return;
     if (t1 < 0) t1 = p.n_tiles;
-    const uint8_t* rec = d_records;
-    if (p.words && reinterpret_cast<uintptr_t>(rec) % 4 != 0)  // a plan built for aligned records
-        fail(STP_INVALID_ARGUMENT, "transpose: genotype records need a 4-byte aligned pitch");
     if (p.detect && detect)
-        launch_detect_ploidy_words(c, rec, p.pitch, p.bpr, p.n_rec, p.n_ind, p.pos.as<int32_t>(), p.sel.as<uint32_t>(), s);
+        launch_detect_ploidy_words(c, d_records, p.pitch, p.bpr, p.n_rec, p.n_ind, p.pos.as<int32_t>(), p.sel.as<uint32_t>(), s);
     if (t1 <= t0) return;
     const bool counts = cnt_ac2 || cnt_packed;
     double* center = is_fx(p.op.fmt) || counts ? nullptr : p.center_ptr + t0 * kTileK;
     const bool early = p.detect && detect;  // the transpose overlaps the ploidy pass
-    launch_transpose_pa(c, rec, p.pitch, p.bpr, p.n_ind, p.tiles.as<TileInfo>() + t0, t1 - t0, p.pos.as<int32_t>(),
+    launch_transpose_pa(c, d_records, p.pitch, p.bpr, p.n_ind, p.tiles.as<TileInfo>() + t0, t1 - t0, p.pos.as<int32_t>(),
                         p.n_sel_pad, p.canon_ptr, center, s, p.row_map.as<int32_t>(), early);
     CanonDecodeArgs a;
     a.canon = p.canon_ptr;
@@ -1925,7 +1919,6 @@ stp_status stp_f2_extract_streamed(stp_ctx* ctx, const stp_f2_request* req, stp_
             c.ws_misc.reserve(operand_plane_bytes(operand_fmt(r.precision, r.n_pop, probe), std::max(r.n_pop, 1), probe.ld));
         }
         std::unique_ptr<Plan> p = build_plan(c, r, dp, c.ws_misc.ptr, true);
-        need(p->words || !r.geno.on_device, "streamed extraction of device records needs a 4-byte aligned pitch");
         if (block_sizes) copy_block_sizes(p->L, block_sizes);
         STPF2_CUDA(cudaStreamSynchronize(c.stream));
         SlabTarget t;

@@ -129,7 +129,13 @@ typedef struct stp_f2_output {
 
 /* ---- context ------------------------------------------------------------------------ */
 
-/* make_cuda_backend(device) (src/device/backend_factory.hpp:18-21). */
+/* make_cuda_backend(device) (src/device/backend_factory.hpp:18-21).
+ *
+ * Device memory: a context keeps workspaces that grow to its largest request. What a call
+ * frees beyond them stays with the library while the device has a context, for the next
+ * call: at most 4 GiB per device, and at most a sixteenth of the device's free memory as it
+ * was when the library last allocated. All of it goes back to the device when an allocation
+ * of the library's would otherwise fail and when the device's last context is destroyed. */
 stp_ctx* stp_create(int device, stp_status* status);
 void stp_destroy(stp_ctx* ctx);
 /* Message of the calling thread's last failed call ("" if none). */

@@ -20,6 +20,7 @@ struct Store {
     std::mutex mu;
     std::vector<Block> blocks[kMaxDevices];
     size_t held[kMaxDevices] = {};
+    size_t limit[kMaxDevices] = {};  // of held, from the last look at the device's memory
     int contexts[kMaxDevices] = {};
 };
 
@@ -38,6 +39,18 @@ size_t rounded(size_t n) {
     size_t r = 512;
     while (r < n) r *= 2;
     return r;
+}
+
+// The blocks released longest ago go until at most `bytes` are held: those of earlier calls of
+// other sizes would otherwise fill the store and every later call allocate anew.
+void trim(Store& s, int device, size_t bytes) {
+    std::vector<Block>& v = s.blocks[device];
+    size_t old = 0;
+    while (s.held[device] > bytes) {
+        s.held[device] -= v[old].bytes;
+        cudaFree(v[old++].p);
+    }
+    v.erase(v.begin(), v.begin() + static_cast<std::ptrdiff_t>(old));
 }
 
 void empty(Store& s, int device) {
@@ -76,7 +89,27 @@ void* pool_alloc(size_t& bytes, int& device) {
         e = cudaMalloc(&p, bytes);
     }
     cuda_check(e, "cudaMalloc");
+    if (known(device)) {
+        // The store holds blocks only while they are a small part of what the device has left
+        // for others: what is held can only grow by a block that was allocated here, so this is
+        // where to look (the query costs less than the allocation it follows).
+        size_t free_b = 0, total = 0;
+        if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
+            (void)cudaGetLastError();
+            free_b = 0;
+        }
+        std::lock_guard<std::mutex> lock(s.mu);
+        s.limit[device] = std::min(kPoolBytes, (free_b + s.held[device]) / kPoolShare);
+        trim(s, device, s.limit[device]);
+    }
     return p;
+}
+
+size_t pool_held(int device) {
+    if (!known(device)) return 0;
+    Store& s = store();
+    std::lock_guard<std::mutex> lock(s.mu);
+    return s.held[device];
 }
 
 void pool_free(void* p, size_t bytes, int device) noexcept {
@@ -87,18 +120,11 @@ void pool_free(void* p, size_t bytes, int device) noexcept {
         cudaDeviceSynchronize() == cudaSuccess) {
         Store& s = store();
         std::lock_guard<std::mutex> lock(s.mu);
-        std::vector<Block>& v = s.blocks[device];
-        if (s.contexts[device] > 0) {
-            // The blocks released longest ago make room: those of earlier calls of other sizes
-            // would otherwise fill the store and every later call allocate anew.
-            size_t old = 0;
-            while (s.held[device] + bytes > kPoolBytes) {
-                s.held[device] -= v[old].bytes;
-                cudaFree(v[old++].p);
-            }
-            v.erase(v.begin(), v.begin() + static_cast<std::ptrdiff_t>(old));
+        const size_t limit = s.limit[device];
+        if (s.contexts[device] > 0 && bytes <= limit / 2) {
+            trim(s, device, limit - bytes);
             try {
-                v.push_back(Block{p, bytes});
+                s.blocks[device].push_back(Block{p, bytes});
                 s.held[device] += bytes;
                 return;
             } catch (...) {

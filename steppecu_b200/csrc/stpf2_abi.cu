@@ -1239,7 +1239,7 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
         size_t free_b = 0, total_b = 0;
         STPF2_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const size_t held = c.ws_batch.bytes + c.ws_f2.bytes + c.ws_vpair.bytes + c.ws_vpc.bytes;  // reusable here
-        const size_t avail = free_b + held;
+        const size_t avail = free_b + held + pool_held(c.device);
         budget = avail > (size_t(2) << 30) ? (avail - (size_t(2) << 30)) * 9 / 10 : 0;
     }
     std::vector<std::vector<size_t>> waves(1);

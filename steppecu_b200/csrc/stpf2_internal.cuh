@@ -47,12 +47,14 @@ inline void cuda_check(cudaError_t e, const char* what) {
 // cudaMalloc / cudaFree of them cost several times the call's kernels (5 of 7.5 ms for the
 // keep mask of 200 populations x 600,000 SNPs). Like cudaFree, pool_free waits for the device
 // before the block can be handed out again, so a block never has work in flight on any
-// stream; the store holds at most kPoolBytes per device (the blocks released longest ago make
-// room), is emptied when an allocation fails and when the device's last context goes, and is
-// guarded by one lock.
+// stream; the store holds at most kPoolBytes per device, and at most one part in kPoolShare of
+// what the device has free (the blocks released longest ago make room), is emptied when an
+// allocation fails and when the device's last context goes, and is guarded by one lock.
 constexpr size_t kPoolBytes = size_t(4) << 30;
+constexpr size_t kPoolShare = 16;
 void* pool_alloc(size_t& bytes, int& device);  // rounds bytes up; raises STP_DEVICE_OOM
 void pool_free(void* p, size_t bytes, int device) noexcept;
+size_t pool_held(int device);  // bytes that an allocation could have as well as the free ones
 void pool_open(int device);   // a context on this device
 void pool_close(int device);  // and its end: the last one empties the store
 

@@ -475,15 +475,35 @@ void copy_block_sizes(const BlockLayout& L, int32_t* out) {
     for (int b = 0; b < L.n_block; ++b) out[b] = L.blocks[b].k;
 }
 
-// Copies record rows [s0, s0 + n) from the host into d, at the records' own pitch hp, on
-// stream st: one contiguous copy (the last row only up to bytes_per_record, which is all a
-// host buffer is sure to hold). Rows of any pitch go as they are: a row-by-row copy into an
-// aligned pitch ran at 4 GB/s for 375-byte rows, the contiguous one at the link's 50.
-void upload_rows(const stp_geno_view& g, uint8_t* d, uint64_t hp, int64_t s0, int64_t n, cudaStream_t st) {
+// Device pitch of host records: their own where one contiguous copy takes them over, that is
+// for rows of whole words, for rows with at most kRowGap bytes between them and for pitches of
+// at most kRowShort; else the record rounded up to 16. A copy row by row moves the records
+// alone, but at 4 to 30 GB/s where the rows lie close (pinned rows of 370 bytes, 100,000 of
+// them, at a pitch of 371: the extraction 12.4 ms, 2.3 contiguous; at 463: 4.6 and 2.3) and never
+// at more than a row in about 10 ns (51 bytes at 409: equal). Further apart it runs at the
+// link's rate, and the contiguous copy would move the gaps too (2,500 bytes at 3,125: 3.3 and 4.0
+// ms; at 20,001: 3.4 and 22.3) and need their room on the device.
+constexpr uint64_t kRowGap = 128, kRowShort = 512;
+uint64_t device_pitch(const stp_geno_view& g) {
+    const uint64_t hp = g.pitch ? g.pitch : g.bytes_per_record;
+    if (hp % 4 == 0 || hp <= std::max(g.bytes_per_record + kRowGap, kRowShort)) return hp;
+    return (g.bytes_per_record + 15) / 16 * 16;
+}
+
+// Copies record rows [s0, s0 + n) from the host into d (pitch dp, device_pitch's) on stream st:
+// one contiguous copy where the pitches agree (the last row only up to bytes_per_record, which
+// is all a host buffer is sure to hold), else row by row.
+void upload_rows(const stp_geno_view& g, uint8_t* d, uint64_t dp, int64_t s0, int64_t n, cudaStream_t st) {
     if (n <= 0) return;
-    const size_t bytes = static_cast<size_t>(n - 1) * hp + std::min(hp, g.bytes_per_record);
-    STPF2_CUDA(cudaMemcpyAsync(d + s0 * static_cast<int64_t>(hp), g.records + s0 * static_cast<int64_t>(hp), bytes,
-                               cudaMemcpyHostToDevice, st));
+    const uint64_t hp = g.pitch ? g.pitch : g.bytes_per_record;
+    uint8_t* to = d + s0 * static_cast<int64_t>(dp);
+    const uint8_t* from = g.records + s0 * static_cast<int64_t>(hp);
+    if (hp == dp)
+        STPF2_CUDA(cudaMemcpyAsync(to, from, static_cast<size_t>(n - 1) * hp + std::min(hp, g.bytes_per_record),
+                                   cudaMemcpyHostToDevice, st));
+    else
+        STPF2_CUDA(cudaMemcpy2DAsync(to, dp, from, hp, g.bytes_per_record, static_cast<size_t>(n),
+                                     cudaMemcpyHostToDevice, st));
 }
 
 // Runs f(i) for i in [0, n) on up to hardware_concurrency threads; rethrows the first error.
@@ -889,10 +909,11 @@ void extract_one(Ctx& c, const stp_f2_request& r, stp_f2_output& o) {
     uint64_t dp = 0;
     if (host_in) {
         need(r.geno.records != nullptr, "records is NULL");
-        dp = pitch;
+        dp = device_pitch(r.geno);
         c.ws_records.reserve(static_cast<size_t>(dp) * r.geno.n_snp);
         if (!pipelined) upload_rows(r.geno, c.ws_records.as<uint8_t>(), dp, 0, r.geno.n_snp, s);
         d_rec = c.ws_records.as<uint8_t>();
+        pitch = dp;
     }
     // A repeated request reuses its plan (whose operand planes already sit in the
     // workspace); otherwise the operand planes borrow the context's grow-only workspace.
@@ -1039,13 +1060,14 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
     need(n_ind > 0, "n_ind must be positive");
     need(g.bytes_per_record > 0, "bytes_per_record is 0");
     need(M < INT_MAX, "too many SNPs");
-    const uint64_t pitch = g.pitch ? g.pitch : g.bytes_per_record;
+    uint64_t pitch = g.pitch ? g.pitch : g.bytes_per_record;
     need(pitch >= g.bytes_per_record, "pitch < bytes_per_record");
     const int prec = reqs[idx[0]].precision;
     const OpFmt fmt = fmt_of(prec);
 
     const uint8_t* d_rec = g.records;
     if (!g.on_device) {
+        pitch = device_pitch(g);
         c.ws_records.reserve(static_cast<size_t>(pitch) * M);
         upload_rows(g, c.ws_records.as<uint8_t>(), pitch, 0, M, s);
         d_rec = c.ws_records.as<uint8_t>();
@@ -1444,6 +1466,7 @@ stp_status stp_decode_counts(stp_ctx* ctx, const stp_geno_view* geno, const int6
         uint64_t pitch = geno->pitch ? geno->pitch : geno->bytes_per_record;
         DevBuf rec;
         if (!geno->on_device) {
+            pitch = device_pitch(*geno);
             rec.reserve(static_cast<size_t>(pitch) * geno->n_snp);
             upload_rows(*geno, rec.as<uint8_t>(), pitch, 0, geno->n_snp, s);
             d_rec = rec.as<uint8_t>();
@@ -1520,6 +1543,7 @@ stp_status stp_snp_keep_mask(stp_ctx* ctx, const stp_geno_view* geno, const int6
             uint64_t pitch = geno->pitch ? geno->pitch : geno->bytes_per_record;
             DevBuf rec;
             if (!geno->on_device) {
+                pitch = device_pitch(*geno);
                 rec.reserve(static_cast<size_t>(pitch) * M);
                 upload_rows(*geno, rec.as<uint8_t>(), pitch, 0, M, s);
                 d_rec = rec.as<uint8_t>();
@@ -1909,8 +1933,9 @@ stp_status stp_f2_extract_streamed(stp_ctx* ctx, const stp_f2_request* req, stp_
         need(pitch >= r.geno.bytes_per_record, "pitch < bytes_per_record");
         need(r.geno.records != nullptr || r.geno.n_snp == 0, "records is NULL");
         uint8_t* d_rec = const_cast<uint8_t*>(r.geno.records);
-        const uint64_t dp = pitch;
+        uint64_t dp = pitch;
         if (!r.geno.on_device && r.geno.n_snp > 0) {
+            dp = device_pitch(r.geno);
             c.ws_records.reserve(static_cast<size_t>(dp) * r.geno.n_snp);
             d_rec = c.ws_records.as<uint8_t>();
         }

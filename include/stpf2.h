@@ -180,7 +180,7 @@ stp_status stp_decode_counts(stp_ctx* ctx, const stp_geno_view* geno, const int6
  * exits), whose address the library takes once per device
  * (cudaGetSymbolAddress) on the first call; make that first call before any stream
  * capture. A request needing more scratch than that (about n_sel * n_snp / 4 bytes of
- * canonical genotypes plus 12 bytes per SNP) fails with STP_INVALID_ARGUMENT. The call
+ * canonical genotypes plus 4 bytes per SNP) fails with STP_INVALID_ARGUMENT. The call
  * sets the scratch that must start at a fixed value (file-row map, error flag) itself.
  * Calls share the scratch: calls on one device that overlap in time (other threads or
  * streams) race and must be serialised by the caller. Work runs on `stream` (NULL = the

@@ -100,7 +100,6 @@ size_t noalloc_scratch_bytes(int64_t n_snp, int64_t n_ind, int64_t n_sel, int P,
     b += round256(static_cast<size_t>(P + 1) * 4);                      // pop_offsets (int32)
     b += round256(static_cast<size_t>(n_tiles) * sizeof(TileInfo));    // tiles
     b += round256(static_cast<size_t>(n_tiles) * kTileK * 4);           // column -> SNP
-    b += round256(static_cast<size_t>(n_tiles) * kTileK * 8);           // column centres
     b += round256(static_cast<size_t>(n_quads) * n_sel_pad * 32);       // canonical quads
     b += 256;                                                            // error flag
     return b;
@@ -115,7 +114,7 @@ void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, uin
         fail(STP_INVALID_ARGUMENT, "no-alloc decode: this request needs " + std::to_string(need) +
                                        " bytes of scratch; the static scratch holds " +
                                        std::to_string(kNoAllocScratchBytes) +
-                                       " (about n_sel * n_snp / 4 bytes of canonical genotypes + 12 bytes per SNP)");
+                                       " (about n_sel * n_snp / 4 bytes of canonical genotypes + 4 bytes per SNP)");
     uint8_t* base = static_cast<uint8_t*>(scratch_base(c.device));
     const int64_t n_tiles = (n_snp + kTileK - 1) / kTileK;
     const int64_t n_quads = (n_tiles + 3) / 4;
@@ -135,7 +134,6 @@ void noalloc_decode_counts(Ctx& c, const uint8_t* d_records, uint64_t pitch, uin
     auto* d_po32 = reinterpret_cast<int32_t*>(take(static_cast<size_t>(P + 1) * 4));
     auto* d_tiles = reinterpret_cast<TileInfo*>(take(static_cast<size_t>(n_tiles) * sizeof(TileInfo)));
     auto* d_col_snp = reinterpret_cast<int32_t*>(take(static_cast<size_t>(n_tiles) * kTileK * 4));
-    auto* d_center = reinterpret_cast<double*>(take(static_cast<size_t>(n_tiles) * kTileK * 8));
     auto* d_canon = reinterpret_cast<uint64_t*>(take(static_cast<size_t>(n_quads) * n_sel_pad * 32));
     auto* d_err = reinterpret_cast<int*>(take(256));
 

@@ -365,12 +365,14 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     p->n_sel_pad = (n_sel + 3) / 4 * 4;
     {
         const size_t canon_bytes = std::max<size_t>(static_cast<size_t>((p->n_tiles + 3) / 4) * p->n_sel_pad * 32, 64);
-        const size_t center_bytes = std::max<size_t>(static_cast<size_t>(p->L.ld) * 8, 64);
         DevBuf& cb = borrow_ws ? c.ws_canon : p->canon;
-        DevBuf& eb = borrow_ws ? c.ws_center : p->center;
         cb.reserve(canon_bytes);
-        eb.reserve(center_bytes);
         p->canon_ptr = cb.as<uint64_t>();
+    }
+    const OpFmt fmt = operand_fmt(r.precision, r.n_pop, p->L);
+    if (!counts_only && !is_fx(fmt)) {  // the operands that are centred
+        DevBuf& eb = borrow_ws ? c.ws_center : p->center;
+        eb.reserve(std::max<size_t>(static_cast<size_t>(p->L.ld) * 8, 64));
         p->center_ptr = eb.as<double>();
     }
 
@@ -381,7 +383,6 @@ std::unique_ptr<Plan> build_plan(Ctx& c, const stp_f2_request& r, uint64_t pitch
     // A plan cached on the context borrows the shared planes workspace, so building another
     // plan there drops it.
     if (planes_base && planes_base == c.ws_misc.ptr) c.plan_cache.reset();
-    const OpFmt fmt = operand_fmt(r.precision, r.n_pop, p->L);
     if (is_fx(fmt) && fx_table_entries(n_max) > 0) {
         p->fx_table.reserve(static_cast<size_t>(fx_table_entries(n_max)) * sizeof(uint2));
         launch_fx_table(c, p->rec_n.as<double>(), p->rec_nm1.as<double>(), n_max, p->fx_table.as<uint2>(), s);
@@ -1110,7 +1111,7 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
     const size_t o_tiles = pa.add(static_cast<size_t>(n_utiles) * sizeof(TileInfo));
     const size_t o_cols = pa.add(static_cast<size_t>(n_utiles) * kTileK * 4);
     const size_t o_canon = pa.add(static_cast<size_t>((n_utiles + 3) / 4) * n_u_pad * 32);
-    const size_t o_center = pa.add(static_cast<size_t>(n_utiles) * kTileK * 8);
+    const size_t o_center = pa.add(fmt == OpFmt::FX ? 0 : static_cast<size_t>(n_utiles) * kTileK * 8);
     const size_t o_t0 = pa.add(16);
     c.pin_union.reserve(staged_a);
     c.ws_union.reserve(pa.end);
@@ -1128,7 +1129,7 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
     auto* d_tiles_u = reinterpret_cast<TileInfo*>(U + o_tiles);
     auto* d_cols_u = reinterpret_cast<int32_t*>(U + o_cols);
     auto* d_canon_u = reinterpret_cast<uint64_t*>(U + o_canon);
-    auto* d_center_u = reinterpret_cast<double*>(U + o_center);
+    auto* d_center_u = fmt == OpFmt::FX ? nullptr : reinterpret_cast<double*>(U + o_center);
     auto* d_t0 = reinterpret_cast<unsigned long long*>(U + o_t0);
 
     launch_timestamp(c, d_t0, s);
@@ -1136,7 +1137,7 @@ void extract_batch_grouped(Ctx& c, const stp_f2_request* reqs, stp_f2_output* ou
                          n_utiles * kTileK, d_cols_u, d_tiles_u, s);
     if (any_auto) launch_detect_ploidy_words(c, d_rec, pitch, g.bytes_per_record, M, n_ind, d_pos_u, d_desc_u, s);
     launch_transpose_pa(c, d_rec, pitch, g.bytes_per_record, n_ind, d_tiles_u, n_utiles, d_pos_u, n_u_pad, d_canon_u,
-                        fmt == OpFmt::FX ? nullptr : d_center_u, s);
+                        d_center_u, s);
 
     // Host tables of every request, in parallel, while the device runs the shared passes.
     std::vector<BatchMember> mem(idx.size());

@@ -170,10 +170,13 @@ void launch_keep_mask_counts(Ctx& c, const uint32_t* cnt, int64_t ld, int P, int
     if (M <= 0) return;
     const unsigned grid = static_cast<unsigned>((M + 255) / 256);
     // The terms of populations of up to 15 samples are 16 KB at most: eight CTAs of 256
-    // threads still fit an SM, and a CTA's table is a small part of the counts it walks when
-    // there are several populations.
+    // threads still fit an SM. A thread computes entries / 256 of them and saves a division per
+    // population, so the table pays from about one population per 128 entries on (600,000 SNPs,
+    // on the fly and table, us: 15 samples 16.1 and 18.2 at 12 populations, 19.2 and 20.1 at 16, 34.0
+    // and 28.9 at 32; 10 samples 13.2 and 13.5 at 8, 16.2 and 15.6 at 12; 5 samples 10.0 and 10.0
+    // at 4, 12.0 and 11.3 at 6; one sample 11.0 and 11.2 at 1, 11.5 and 10.9 at 4).
     const int64_t entries = n_max <= 31 ? (n_max + 1) * (2 * n_max + 1) : 0;
-    if (entries > 0 && P >= 8)
+    if (entries > 0 && P >= 3 + entries / 128)
         keep_mask_counts_kernel<true><<<grid, 256, static_cast<size_t>(entries) * sizeof(double), s>>>(
             cnt, ld, P, M, rec_n, static_cast<int>(n_max), ref, alt, chrom, f, total_indiv, keep, out4);
     else

@@ -1,5 +1,5 @@
-"""The keep mask's terms from the shared table (populations of up to 15 samples, eight or more
-of them) and on the fly (either side of both lines): the same sums as the oracle, bit for bit."""
+"""The keep mask's terms from the shared table (populations of up to 15 samples, enough of them
+for the table's size) and on the fly (either side of both lines): the same sums as the oracle, bit for bit."""
 from __future__ import annotations
 
 import numpy as np
@@ -10,7 +10,8 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("P,largest", [(7, 15), (8, 1), (8, 15), (8, 16), (41, 15), (200, 3)])
+@pytest.mark.parametrize("P,largest", [(7, 15), (8, 1), (8, 15), (8, 16), (41, 15), (200, 3),
+                                       (17, 15), (18, 15), (9, 10), (10, 10), (4, 5), (5, 5), (2, 1), (3, 1)])
 @pytest.mark.parametrize("n_snp", [1, 257, 1000])
 def test_pooled_sums_bitexact(ctx, P, largest, n_snp):
     rng = np.random.default_rng(P * 100 + largest + n_snp)

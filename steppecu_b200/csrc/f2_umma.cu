@@ -6,10 +6,12 @@
 //   warp 0      producer: per 32-SNP stage, bulk-copies the pre-swizzled operand image of
 //               the row tile and of the column tile (one side on diagonal tiles): 44 KiB
 //               each, the 5 split planes (Pt_hi, Pt_lo, Ah_hi, Ah_lo, M as 16-bit) and the
-//               int8 M plane in one contiguous copy; no tensor maps, no multicast.
-//   warp 1      TMEM owner + single-thread tcgen05.mma issuer. Per 16-SNP K step, seven
-//               kind::f16 MMAs accumulate num/2 = sum(Ah_i M_j + M_i Ah_j - Pt_i Pt_j) over
-//               the hi/lo splits (the -Pt Pt products use the descriptor's A-negate bit)
+//               int8 M plane in one contiguous copy (the valid rows of a side that is not
+//               whole in six); no tensor maps, no multicast.
+//   warp 1      TMEM owner + tcgen05.mma issuer (the whole warp, one elected lane around the
+//               MMAs). Per 16-SNP K step, seven kind::f16 MMAs accumulate
+//               num/2 = sum(Ah_i M_j + M_i Ah_j - Pt_i Pt_j) over the
+//               hi/lo splits (the -Pt Pt products use the descriptor's A-negate bit)
 //               into one FP32 TMEM buffer per chunk (64 SNPs = two stages; 32 SNPs in the
 //               fine mode); one kind::i8 MMA per stage
 //               accumulates the exact both-present count M M^T into an int32 TMEM buffer.
@@ -147,15 +149,16 @@ __device__ __forceinline__ int read_item(const UmmaArgs& a, SmemCtl* ctl, uint32
     return it;
 }
 
-// A tile side with few populations: the 8-row groups a stage copies of it (all 16 in one copy,
-// or, up to half of them, the valid ones of each plane in six copies), and the MMA columns of
-// a column tile (its populations rounded up to 16). Rows and columns past the valid ones make
+// A tile side with fewer than 128 populations: the 8-row groups a stage copies of it (a whole
+// side in one copy, else the valid ones of each plane in six copies), and the MMA columns of a
+// column tile (its populations rounded up to 16). Rows and columns past the valid ones make
 // accumulators that nothing reads, whatever the slot held there. 300 populations leave a last
-// tile of 44, and half of their tile pairs meet it: the kernel 809 -> 744 us.
-__device__ __forceinline__ uint32_t side_groups(int rows) {
-    const uint32_t g = static_cast<uint32_t>((rows + 7) / 8);
-    return g <= 8 ? g : 16u;
-}
+// tile of 44, and half of their tile pairs meet it: the kernel 809 -> 744 us. Six copies beat
+// one up to 15 groups (200,000 SNPs in 140 blocks, one tile, all rows and valid rows, us: 8
+// populations 55.8 and 36.8, 64 66.5 and 52.8, 72 68.4 and 57.2, 96 68.8 and 61.9, 104 70.4 and
+// 66.1, 120 71.3 and 69.5; as the last of three tiles 305 and 290 at 8, 340 and 335 at 96, 351 and
+// 350 at 120).
+__device__ __forceinline__ uint32_t side_groups(int rows) { return static_cast<uint32_t>((rows + 7) / 8); }
 __device__ __forceinline__ uint32_t side_bytes(uint32_t g) { return g == 16 ? kSideBytes : g * (kPlanes * 512u + 256u); }
 __device__ __forceinline__ void copy_side(uint8_t* dst, const uint8_t* img, uint32_t g, unsigned long long* bar) {
     if (g == 16) {

@@ -23,7 +23,7 @@ BOUND = {mode: 8 * u * u + 28 * 2.0**-23 for mode, u in ROUNDOFF.items()}
 
 
 @pytest.mark.parametrize("mode", list(BOUND))
-@pytest.mark.parametrize("P", [1, 8, 9, 31, 33, 64, 65, 128, 129, 150, 192, 300])
+@pytest.mark.parametrize("P", [1, 8, 9, 31, 33, 64, 65, 72, 97, 120, 121, 128, 129, 150, 192, 233, 300])
 def test_split_tiles_match_oracle(ctx, mode, P):
     p = synth.generate("c4", seed=40 + P, n_snp=sum(SIZES), n_pop=P)
     sel, po = p.selection()

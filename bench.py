@@ -3,18 +3,23 @@
 Metric: f2 SNP-pop-pairs/s = M * P*(P-1)/2 per extraction pass, per second. A step is one
 pass of the hot path (ploidy -> decode -> per-block contraction -> FP64 f2/vpair) over
 one synthetic panel already resident in HBM. Workload (default): 1,000 populations x 10
-samples (10,000 total), 1,150,000 SNPs on 22 chromosomes, 5 cM blocks (~700), split-F16
-tensor-core contraction (split-BF16 and the plain FP32 SIMT form are timed beside it). The panel (2.9 GB of genotypes, ~12 GB of operands) is far larger
-than L2, so no flush is needed between steps.
+samples (10,000 total), 1,150,000 SNPs on 22 chromosomes, 5 cM blocks (~700), the fixed-point
+tensor-core contraction (the split forms and the plain FP32 SIMT form are timed beside it). The
+panel (2.9 GB of genotypes, ~10 GB of operands) is far larger than L2, so no flush is needed
+between steps.
 
 `e2e` times the same extraction through the C ABI with host buffers: pinned genotypes in,
 H2D copy, extraction, D2H of the FP64 f2 and vpair tensors, every step.
 
 `--impl reference` times the reference's own CpuBackend (oracle/_ref, built from the
-reference sources; the C restatement when that is absent) on the host cores, one
-jackknife block per thread, on a bounded sample of the same workload. The same sample is
-extracted on the GPU in every arithmetic and compared with it: `precision` reports the
-max abs / rel f2 error against the reference at the workload's full population count.
+reference sources) on the host cores, one jackknife block per thread, on a bounded sample of
+the same workload; without that build it prints an `unavailable` line. The default arm runs the
+same sample as `cpu_baseline` (there by the C restatement when the reference's build is absent:
+its `kind` says which), extracts it on the GPU in every arithmetic and compares:
+`max_abs_error` is the largest f2 error of each at the workload's full population count.
+
+The printed line carries the figures of each part; everything measured (per-block errors, every
+configuration's split, the samples' descriptions) goes to the file of `--detail`.
 
 Multi-GPU (torchrun): blocks are independent, so every rank extracts its own panel (a
 different genome segment of the same shape): weak scaling, no data-path collective.
@@ -336,9 +341,52 @@ def precision_report(ctx, sample, modes) -> dict:
     return out
 
 
+def rounded(x, digits: int = 6):
+    """x with every float at `digits` significant digits."""
+    if isinstance(x, dict):
+        return {k: rounded(v, digits) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [rounded(v, digits) for v in x]
+    return float(f"{x:.{digits}g}") if isinstance(x, float) else x
+
+
+def headline(line: dict) -> dict:
+    """The line to print from everything measured: the run's own figures whole, one number per
+    part of the rest. Kept short (about 2,000 characters), so that it survives readers that
+    keep the end of a log only."""
+    def pick(d, keys):
+        return None if d is None else {k: d[k] for k in keys if k in d}
+
+    out = {k: v for k, v in line.items() if k not in (
+        "e2e", "roofline", "cpu_baseline", "precision", "precision_all_blocks", "other_arithmetics", "per_block_launches",
+        "fstats", "batched_requests", "other_configs", "value_ordered_pairs")}
+    out["e2e"] = pick(line["e2e"], ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_step", "steps"))
+    out["roofline"] = pick(line["roofline"], ("bound", "achieved", "peak", "unit", "frac", "traffic", "peak_source",
+                                              "kernel_ms", "decode_ms", "decode_hbm_gbs"))
+    out["cpu_baseline"] = pick(line["cpu_baseline"], ("value", "unit", "cores", "kind"))
+    prec = line["precision"]
+    out["max_abs_error"] = prec if prec is None else {k: v if k == "against" else v["max_abs"] for k, v in prec.items()}
+    out["precision_all_blocks"] = pick(line["precision_all_blocks"], ("blocks", "max_abs", "tolerance", "vpair_bit_exact"))
+    out["other_arithmetics_ms"] = {k: v["ms_per_step"] for k, v in (line["other_arithmetics"] or {}).items()}
+    out["per_block_launches_ms"] = line["per_block_launches"] and line["per_block_launches"]["ms_per_step"]
+    out["fstats_ms"] = line["fstats"] and line["fstats"]["ms"]
+    b = line["batched_requests"]
+    out["batched_requests"] = b and pick(b["grouped"], ("value", "ms_per_call", "device_span_ms", "equals_serial"))
+    out["other_configs_ms"] = line["other_configs"] and {
+        c: {m: v["ms_per_step"] for m, v in d.items() if isinstance(v, dict) and "ms_per_step" in v}
+        for c, d in line["other_configs"].items()}
+    return rounded(out)
+
+
 def run_reference(args, rank: int, world: int):
     threads = os.cpu_count() or 1
     if rank != 0:
+        return
+    import oracle
+
+    if not oracle.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not present, so its CpuBackend "
+                                                              "is not built (oracle/_ref)"}), flush=True)
         return
     for _ in range(args.warmup):
         cpu_sample(args.workload, threads)
@@ -586,6 +634,8 @@ def main():
                     help="per-block f2 error of the headline pass against the CPU oracle on the pairs of every "
                          "n-th population, all blocks (1: all pairs, several minutes of host time at 1,000 "
                          "populations; 0: skip)")
+    ap.add_argument("--detail", type=Path, default=ROOT / "_build" / "bench_detail.json",
+                    help="file for everything measured (default: %(default)s)")
     args = ap.parse_args()
 
     rank = int(os.environ.get("RANK", "0"))
@@ -819,7 +869,9 @@ def main():
             "batched_requests": batched,
             "other_configs": other_configs,
         }
-        print(json.dumps(line), flush=True)
+        args.detail.parent.mkdir(parents=True, exist_ok=True)
+        args.detail.write_text(json.dumps(line, indent=1))
+        print(json.dumps(headline(line)), flush=True)
     if batched is None:
         plan.close()
         ctx.close()

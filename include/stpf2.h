@@ -367,7 +367,11 @@ stp_status stp_plan_run(stp_plan* plan, const uint8_t* d_records, double* d_f2, 
 stp_status stp_plan_run_graph(stp_plan* plan, const uint8_t* d_records, double* d_f2, double* d_vpair,
                               void* stream);
 /* Comparison form of the contraction (tensor-core plans): one launch per jackknife block
- * instead of one persistent launch over every block's tile pairs. Same results. */
+ * instead of one persistent launch over every block's tile pairs. Same results; with
+ * STP_PREC_FIXED_I8 and up to 64 populations the two forms run different kernels, whose f2
+ * agrees bit for bit for blocks of up to 16,384 SNPs and to rounding beyond, and the switch
+ * rebuilds the plan's operands: it may fail with STP_DEVICE_OOM, and the plan then stays as
+ * it was. */
 stp_status stp_plan_set_per_block_launch(stp_plan* plan, int32_t enable);
 /* Kernel launches one stp_plan_run issues. */
 int32_t stp_plan_launches(const stp_plan* plan);

@@ -1,8 +1,10 @@
 // steppecu_b200/csrc/f2_fxs.cu
 //
 // The fixed-point f2 contraction of f2_fx.cu for requests of at most 64 populations: the same
-// digits, the same exact integer sums and the same result (f2_fx.cu's header has the
-// arithmetic), with the digit planes stacked into the MMA's rows and columns.
+// digits and exact integer sums (f2_fx.cu's header has the arithmetic), with the digit planes
+// stacked into the MMA's rows and columns. A block's sum is one int64 here and rounded once; the
+// general kernel rounds and adds in FP64 per 16,384 SNPs. So the results are the same bit for
+// bit for blocks of up to 16,384 SNPs, and within a few FP64 roundings beyond.
 //
 // With P <= 64 populations a 128-row tile of one plane is mostly padding, and an MMA of N <=
 // 64 columns costs as much as one of 64 (about 44 cycles whatever its columns), so the
@@ -21,16 +23,20 @@
 //     T_hi(i, j) = 2 [X3X0 + M E3 + 2^8 (X3X1 + M E4) + 2^16 (X3X2 + M E5)] + 2^24 X3X3
 //     T_lo(i, j) = 2 [X2X1 + 2^24 E6 M] + 2^8 X2X2
 //     W(i, j)    = (T(i, j) + T(j, i)) / 2,   T = T_hi + T_lo
-// and W is f2_fx_kernel's W: |T| < 2^39.6 per SNP, so int64 holds a block of 2^22 SNPs (longer
-// blocks take the general kernels). An accumulator entry is one digit product per SNP, at
+// and W is f2_fx_kernel's W, over the whole block: |T| < 2^39.6 per SNP, so int64 holds a block
+// of 2^22 SNPs (longer blocks take the general kernels). An accumulator entry is one digit product per SNP, at
 // most 2^14, so int32 holds 131,040 SNPs; longer blocks run in segments.
 //
 // One persistent launch, one CTA per SM: warp 0 copies (several chunks per bulk copy: the
 // images of consecutive chunks are contiguous), warp 1 issues the MMAs, eight epilogue warps
 // read the accumulators, exchange T through shared memory and write whole slabs of f2 and
 // vpair as contiguous runs. Up to 32 rows per plane two accumulators alternate; above, one.
-// Measured (f2 and counts together): 20 populations x 50,000 SNPs in 40 blocks 32.4 -> 10.3 us; the sixteen
-// requests of 4 to 64 populations in a batch over 400,000 SNPs 1,612 -> 366 us.
+// Measured (f2 and counts together): 20 populations x 50,000 SNPs in 40 blocks 32.4 -> 10.3 us; the
+// sixteen requests of 4 to 64 populations in a batch over 400,000 SNPs 1,612 -> 366 us. The line at
+// 64 is where the planes fill the accumulators; up to it the stacked form is the faster one alone
+// too (whole passes over 200,000 SNPs in 140 blocks, general and stacked: 33 populations 151 and
+// 58 us, 48 163 and 68, 64 164 and 80; over one block 5.8 ms and 0.9 to 1.3; 10,000 blocks of 10
+// SNPs 1.03 ms and 0.32 to 0.57), while 65 populations take the general one (122 us).
 #include <algorithm>
 
 #include "stpf2_internal.cuh"

@@ -1684,7 +1684,7 @@ stp_status stp_decode_counts_noalloc(stp_ctx* ctx, const stp_geno_view* geno, co
         need(geno->records && pop_offsets && d_ac2 && d_n, "null argument");
         const uint64_t pitch = geno->pitch ? geno->pitch : geno->bytes_per_record;
         need(pitch % 16 == 0 && reinterpret_cast<uintptr_t>(geno->records) % 16 == 0,
-             "the no-alloc decode needs 16-byte aligned records and pitch (it cannot repitch without a buffer)");
+             "the no-alloc decode needs 16-byte aligned records and pitch");
         need(pitch >= geno->bytes_per_record, "pitch smaller than bytes_per_record");
         need(pop_offsets[0] == 0, "pop_offsets[0] must be 0");
         for (int i = 0; i < n_pop; ++i) {

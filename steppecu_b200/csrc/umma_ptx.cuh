@@ -77,9 +77,10 @@ __device__ __forceinline__ bool wait_bounded(unsigned long long* b, uint32_t par
 // moves each over per instruction. So a whole warp runs an issuing role, every value that
 // reaches those instructions made uniform where it enters (uni), and one elected lane executes
 // them, with descriptors that differ by constants from one per slot. Against single-lane roles:
-// f2 at 100 populations x 1.15M SNPs 269 -> 254 us, at 603 ragged ones 1,341 -> 1,294; their
-// counts 133 -> 114; the split form at 300 x 400,000 832 -> 809. At 1,000 populations the tensor
-// and shared-memory pipes bound f2 and it stays where it was.
+// f2 at 100 populations x 1.15M SNPs 269 -> 254 us, at 603 ragged ones 1,341 -> 1,283; their
+// counts 133 -> 114; the split form at 300 x 400,000 832 -> 809. At 1,000 populations, where the
+// tensor and shared-memory pipes bound f2, 8.76 -> 8.48 ms (the fastest launches; 9.4 -> 9.0 in
+// the median, under the power cap), and the counts 0.81 -> 0.72.
 __device__ __forceinline__ int uni(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 __device__ __forceinline__ uint32_t uni(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
 __device__ __forceinline__ int64_t uni(int64_t x) { return __shfl_sync(0xffffffffu, x, 0); }

@@ -108,9 +108,9 @@ def test_fixed_i8_long_blocks_span_accumulator_segments(ctx, out_on_device):
 
 
 def test_fixed_i8_block_longer_than_one_count_accumulation(ctx):
-    """A block of 530,000 SNPs: the vpair kernel's int32 accumulator holds 524,032 SNPs of
-    64 x 64 products, so the block's counts come from two accumulations (and its f2 from 33
-    segments of 16,384 SNPs); a short block follows."""
+    """A block of 530,000 SNPs, at few populations (the stacked kernel: five accumulator segments
+    of 131,040 SNPs); a short block follows. test_gpu_fx_general.py has the general kernels'
+    count accumulations of 524,032."""
     p = synth.generate("c1", seed=21, n_snp=531_000, n_pop=9)
     sel, po = p.selection()
     rec = p.records_numpy()
@@ -123,9 +123,9 @@ def test_fixed_i8_block_longer_than_one_count_accumulation(ctx):
 
 
 def test_fixed_i8_wait_timeout_reports_and_context_recovers():
-    """A wait that runs out (the hook stops the f2 kernel's feed) ends the call with
-    STP_DEVICE_TIMEOUT; the kernel frees its tensor memory and exits, and the same context
-    then extracts correctly."""
+    """A wait that runs out (the hook stops the feed; at nine populations the stacked kernel's)
+    ends the call with STP_DEVICE_TIMEOUT; the kernel frees its tensor memory and exits, and the
+    same context then extracts correctly. test_gpu_fx_general.py has the general kernel's."""
     from steppecu_b200 import Context
 
     p = synth.generate("c1", seed=11, n_snp=3000, n_pop=9)
@@ -147,7 +147,8 @@ def test_fixed_i8_wait_timeout_reports_and_context_recovers():
 @pytest.mark.parametrize("P", [41, 150, 250])
 def test_tile_classes_do_not_change_results(ctx, P):
     """The partial-feed tile classes (stp_set_tile_classes) only change which rows a stage
-    copies: every class mask gives the same f2 and vpair, bit for bit."""
+    copies: every class mask gives the same f2 and vpair, bit for bit (41 populations take the
+    stacked kernel, which has no classes; test_gpu_fx_general.py has such a last tile)."""
     p = synth.generate("c4", seed=300 + P, n_snp=20_000, n_pop=P)
     sel, po = p.selection()
     rec = p.records_numpy()

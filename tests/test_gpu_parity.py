@@ -123,10 +123,8 @@ def test_decode_counts_device_records(ctx, uneven):
 @pytest.mark.parametrize("panel_pops,n_snp", [(1232, 4001), (1250, 4000)])
 def test_wide_panel_scattered_selection(ctx, panel_pops, n_snp):
     """40 scattered populations, in descending order, from panels of 12,320 and 12,500
-    samples. 12,320 samples give 3,080-byte records, a multiple of 4 bytes but not of 16,
-    which the transpose reads at their own pitch with 4-byte copies; 12,500 samples give
-    3,125-byte records, which are re-pitched to 16 bytes first. Counts bit-exact, f2 within
-    tolerance."""
+    samples: 3,080-byte records, a multiple of 4 bytes but not of 16, and 3,125-byte ones, off
+    a word, both read in place. Counts bit-exact, f2 within tolerance."""
     p = synth.generate("c3", seed=panel_pops + n_snp, n_snp=n_snp, n_pop=panel_pops)
     sel, po = p.selection(list(range(panel_pops - 1, -1, -31))[:40])
     rec = p.records_numpy()

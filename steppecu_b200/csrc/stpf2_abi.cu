@@ -921,7 +921,7 @@ void extract_one(Ctx& c, const stp_f2_request& r, stp_f2_output& o) {
     std::unique_ptr<Plan> p = take_cached_plan(c, r, pitch);
     const bool hit = p != nullptr;
     if (!hit) {
-        const BlockLayout probe = make_block_layout(r.block_id, snp_axis(r), r.n_block);
+        const BlockLayout probe = make_block_layout(r.block_id, snp_axis(r), r.n_block, false);
         c.ws_misc.reserve(operand_plane_bytes(operand_fmt(r.precision, r.n_pop, probe), std::max(r.n_pop, 1), probe.ld));
         p = build_plan(c, r, pitch, c.ws_misc.ptr, true);
     }
@@ -1941,7 +1941,7 @@ stp_status stp_f2_extract_streamed(stp_ctx* ctx, const stp_f2_request* req, stp_
             d_rec = c.ws_records.as<uint8_t>();
         }
         {
-            const BlockLayout probe = make_block_layout(r.block_id, snp_axis(r), r.n_block);
+            const BlockLayout probe = make_block_layout(r.block_id, snp_axis(r), r.n_block, false);
             c.ws_misc.reserve(operand_plane_bytes(operand_fmt(r.precision, r.n_pop, probe), std::max(r.n_pop, 1), probe.ld));
         }
         std::unique_ptr<Plan> p = build_plan(c, r, dp, c.ws_misc.ptr, true);
